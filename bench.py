@@ -974,7 +974,7 @@ def main():
 
     peaks = load_peaks()
     l2 = l2_read_peak(stream, f"cuda:{local}", ctx_sms(ctx))
-    per_ray_model = 128.0 * nodes_visited / N_RAYS + 48.0 * tris_tested / N_RAYS + 40.0
+    per_ray_model = 64.0 * nodes_visited / N_RAYS + 48.0 * tris_tested / N_RAYS + 40.0
     achieved = per_ray_model * N_RAYS / (ms * 1e-3) / 1e9
     traffic = None
     prof = ROOT / "profiles" / "trace_closest_traffic.json"
@@ -993,7 +993,7 @@ def main():
         "visits_per_ray": {"nodes": nodes_visited / N_RAYS, "triangles": tris_tested / N_RAYS},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"], "traffic": traffic,
-                     "model": "128 B x nodes visited + 48 B x triangles tested + 40 B per ray, counted on device",
+                     "model": "64 B x nodes visited + 48 B x triangles tested + 40 B per ray, counted on device",
                      "peak_source": peaks["source"],
                      "l2": {"peak": l2["gbs"], "frac": achieved / l2["gbs"], "unit": "GB/s",
                             "peak_by_buffer_mib": l2["by_buffer_mib"], "peak_source": l2["source"]}},

@@ -85,14 +85,12 @@ int launch_trace_t(liar_gpu_ctx* ctx, const liar_gpu_mesh* m, const liar_ray* d_
         if (e != cudaSuccess) return ctx_cuda(ctx, e, "occupancy query");
         if (per_sm <= 0) per_sm = 1;
     }
-    const uint64_t needed_blocks = ((uint64_t)n + BLOCK - 1) / BLOCK;
-    uint64_t blocks = (uint64_t)ctx->num_sms * per_sm;
-    if (blocks > needed_blocks) blocks = needed_blocks;
-    if (blocks == 0) blocks = 1;
+    const uint32_t resident = (uint32_t)ctx->num_sms * per_sm * (BLOCK / 32);
+    const uint32_t blocks = (trace_warps(n, resident, (uint32_t)ctx->num_sms) + BLOCK / 32 - 1) / (BLOCK / 32);
     cudaError_t e = cudaMemsetAsync(d_counter, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "reset work counter");
-    const uint32_t batch = trace_batch(n, (uint32_t)blocks * (BLOCK / 32));
-    kern<<<(unsigned)blocks, BLOCK, smem, st>>>(m->d_nodes, m->d_tris, d_rays, d_hits, n, d_counter, d_status,
+    const uint32_t batch = trace_batch(n, blocks * (BLOCK / 32));
+    kern<<<blocks, BLOCK, smem, st>>>(m->d_nodes, m->d_tris, d_rays, d_hits, n, d_counter, d_status,
                                              d_counters, batch, n_dev);
     return ctx_cuda(ctx, cudaGetLastError(), "trace kernel launch");
 }

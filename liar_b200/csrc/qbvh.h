@@ -6,13 +6,17 @@
 // TriangleMesh::doIntersect / doIsIntersecting (src/liar/scenery/triangle_mesh.cpp:291-330).
 // Lass is not part of the reference sources, so the tree here is an own design:
 //
-//   QNode (128 B, one L2 line): the four child boxes as structure-of-arrays float4 rows so
-//   that one thread reads all four boxes with six 16-byte loads, plus the child links.
+//   QNode (64 B, half an L2 line): the four child boxes quantised within the node's own box, the
+//   planes as byte codes q. Code q stands for the float with bits 0x40qq0000, plane_value(q): 2 .. 4
+//   in steps of 1/64 for q < 128, then 4 .. 8 in steps of 1/32, so that a byte becomes a float by a
+//   byte permutation alone. A plane lies at org + plane_value(q) * scl; the builder picks codes
+//   that keep the padded child box inside the decoded one.
+//     org, scl : the grid of each axis
+//     lo, hi   : word a = axis a, byte c = child c
 //     child[c] >= 0 : index of an inner QNode
 //     child[c] <  0 : leaf, packed as 0x80000000 | count << 27 | first, holding the triangles
 //                     tris[first .. first + count) (count <= 8, first < 2^27); count 0 marks an
-//                     empty slot, whose box is also inverted so that it never hits
-//     count[c]      : the leaf's triangle count again (0 for inner nodes), kept for tools
+//                     empty slot, whose box is also inverted on every axis (lo 255, hi 0)
 //
 //   QTri (48 B): v0, e1 = v1 - v0, e2 = v2 - v0 as three float4, the original triangle index in
 //   the w lane of the first; e1.w = 0. A sphere primitive has its centre in v0, its radius in
@@ -33,16 +37,21 @@ namespace liar_gpu {
 struct alignas(16) F4 { float x, y, z, w; };
 struct alignas(16) I4 { int32_t x, y, z, w; };
 
-struct alignas(128) QNode {
-    F4 lo_x, hi_x, lo_y, hi_y, lo_z, hi_z;  // child c bounds in lane c
-    I4 child;                               // see above
-    I4 count;                               // leaf triangle count per child, 0 for inner/empty
+struct alignas(64) QNode {
+    float org[3], scl[3];
+    uint32_t lo[3], hi[3];
+    int32_t child[4];
 };
-static_assert(sizeof(QNode) == 128, "QNode must be one 128-byte line");
-// the traversal selects a child row's near or far plane by these offsets (hi_* = lo_* + 16 bytes)
-static_assert(offsetof(QNode, lo_x) == 0 && offsetof(QNode, hi_x) == 16 && offsetof(QNode, lo_y) == 32 &&
-                  offsetof(QNode, hi_y) == 48 && offsetof(QNode, lo_z) == 64 && offsetof(QNode, hi_z) == 80,
-              "QNode plane rows");
+static_assert(sizeof(QNode) == 64, "QNode must be 64 bytes");
+// the traversal reads the node as four 16-byte rows
+static_assert(offsetof(QNode, scl) == 12 && offsetof(QNode, lo) == 24 && offsetof(QNode, hi) == 36 &&
+                  offsetof(QNode, child) == 48,
+              "QNode rows");
+
+// the float a plane code stands for
+LIAR_HD inline float plane_value(uint32_t q) {
+    return q < 128u ? 2.0f + (float)q * 0.015625f : 4.0f + (float)(q - 128u) * 0.03125f;
+}
 
 struct alignas(16) QTri {
     F4 v0;   // v0.xyz, w = original triangle index (int bits)

@@ -180,9 +180,33 @@ struct Builder {
     }
 };
 
+// f(begin, end) over pieces of [0, n) on up to `threads` threads; small ranges and the pieces of
+// threads that cannot be started run here
+template <class F>
+void in_pieces(size_t n, int threads, const F& f) {
+    const size_t pieces = std::min<size_t>((size_t)std::max(threads, 1), n / 8192 + 1), each = (n + pieces - 1) / pieces;
+    std::vector<std::thread> run;
+    size_t at = each;
+    try {
+        run.reserve(pieces);
+        for (; at < n; at += each) {
+            const size_t end = std::min(n, at + each);
+            run.emplace_back([&f, at, end]() { f(at, end); });
+        }
+    } catch (...) {
+        f(at, n);
+    }
+    f((size_t)0, std::min(n, each));
+    for (std::thread& t : run) t.join();
+}
+
 struct Collapser {
     const std::vector<BNode>& bnodes;
+    struct Members {
+        int32_t b[4];  // binary-tree nodes of the slots, -1 for none
+    };
     std::vector<QNode> qnodes;
+    std::vector<Members> members;
     float pad;
     double root_area;
     double sah = 0.0;
@@ -193,77 +217,125 @@ struct Collapser {
 
     Collapser(const std::vector<BNode>& b, float p, double ra, double ct) : bnodes(b), pad(p), root_area(ra), c_trav(ct) {}
 
-    static float down(float x) { return std::nextafter(x, -INFINITY); }
-    static float up(float x) { return std::nextafter(x, INFINITY); }
+    // the next float below and above (nextafter without the call)
+    static float step(float x, bool up) {
+        if (x == 0.0f) return up ? 1.40129846e-45f : -1.40129846e-45f;
+        int32_t i;
+        std::memcpy(&i, &x, 4);
+        if ((i & 0x7f800000) == 0x7f800000) return x;  // infinities stay
+        i += (i >= 0) == up ? 1 : -1;
+        std::memcpy(&x, &i, 4);
+        return x;
+    }
+    static float down(float x) { return step(x, false); }
+    static float up(float x) { return step(x, true); }
+    // the code whose plane_value is nearest below v (clamped)
+    static int code_of(double v) {
+        const double c = v < 4.0 ? (v - 2.0) * 64.0 : 128.0 + (v - 4.0) * 32.0;
+        return c <= 0.0 ? 0 : c >= 255.0 ? 255 : (int)c;
+    }
 
     // returns the index of the new QNode
     int32_t emit(int32_t bi, uint32_t depth, uint32_t stack_so_far) {
-        std::vector<int32_t> kids;
+        int32_t kids[4];
+        int n_kids = 0;
         const BNode& b = bnodes[bi];
         if (b.left < 0) {
-            kids.push_back(bi);  // a root that is a single leaf
+            kids[n_kids++] = bi;  // a root that is a single leaf
         } else {
-            kids.push_back(b.left);
-            kids.push_back(b.right);
+            kids[n_kids++] = b.left;
+            kids[n_kids++] = b.right;
         }
-        while (kids.size() < 4) {
+        while (n_kids < 4) {
             int pick = -1;
             double pick_area = -1.0;
-            for (size_t k = 0; k < kids.size(); ++k) {
+            for (int k = 0; k < n_kids; ++k) {
                 const BNode& c = bnodes[kids[k]];
                 if (c.left >= 0 && c.box.area() > pick_area) {
                     pick_area = c.box.area();
-                    pick = (int)k;
+                    pick = k;
                 }
             }
             if (pick < 0) break;
             const BNode& c = bnodes[kids[pick]];
             kids[pick] = c.left;
-            kids.push_back(c.right);
+            kids[n_kids++] = c.right;
         }
         const int32_t qi = (int32_t)qnodes.size();
         qnodes.emplace_back();
+        members.emplace_back();
         sah += c_trav * bnodes[bi].box.area() / root_area;
         max_depth = std::max(max_depth, depth + 1);
-        const uint32_t stack_here = stack_so_far + (uint32_t)(kids.size() - 1);
+        const uint32_t stack_here = stack_so_far + (uint32_t)(n_kids - 1);
         max_stack = std::max(max_stack, stack_here);
-        float lo[3][4], hi[3][4];
-        int32_t child[4], count[4];
-        for (int c = 0; c < 4; ++c) {
-            for (int a = 0; a < 3; ++a) {
-                lo[a][c] = INFINITY;
-                hi[a][c] = -INFINITY;
-            }
-            child[c] = (int32_t)0x80000000u;  // empty leaf slot: zero triangles
-            count[c] = 0;
-        }
-        for (size_t k = 0; k < kids.size(); ++k) {
+        int32_t child[4];
+        for (int c = 0; c < 4; ++c) child[c] = (int32_t)0x80000000u;  // empty leaf slot: zero triangles
+        for (int k = 0; k < n_kids; ++k) {
             const BNode& c = bnodes[kids[k]];
-            for (int a = 0; a < 3; ++a) {
-                lo[a][k] = down(c.box.lo[a] - pad);
-                hi[a][k] = up(c.box.hi[a] + pad);
-            }
             if (c.left < 0) {
                 child[k] = (int32_t)(0x80000000u | (c.count << 27) | c.first);
-                count[k] = (int32_t)c.count;
                 sah += (double)c.count * c.box.area() / root_area;
                 ++leaves;
             }
         }
-        for (size_t k = 0; k < kids.size(); ++k) {
+        for (int k = 0; k < n_kids; ++k) {
             const BNode& c = bnodes[kids[k]];
             if (c.left >= 0) child[k] = emit(kids[k], depth + 1, stack_here);
         }
-        QNode& q = qnodes[qi];
-        q.lo_x = {lo[0][0], lo[0][1], lo[0][2], lo[0][3]};
-        q.hi_x = {hi[0][0], hi[0][1], hi[0][2], hi[0][3]};
-        q.lo_y = {lo[1][0], lo[1][1], lo[1][2], lo[1][3]};
-        q.hi_y = {hi[1][0], hi[1][1], hi[1][2], hi[1][3]};
-        q.lo_z = {lo[2][0], lo[2][1], lo[2][2], lo[2][3]};
-        q.hi_z = {hi[2][0], hi[2][1], hi[2][2], hi[2][3]};
-        q.child = {child[0], child[1], child[2], child[3]};
-        q.count = {count[0], count[1], count[2], count[3]};
+        for (int c = 0; c < 4; ++c) {
+            qnodes[qi].child[c] = child[c];
+            members[qi].b[c] = c < n_kids ? kids[c] : -1;
+        }
         return qi;
+    }
+
+    // the quantised boxes of node qi, from its members' boxes
+    void quantise(size_t qi) {
+        QNode& q = qnodes[qi];
+        const int32_t* kids = members[qi].b;
+        int n_kids = 0;
+        while (n_kids < 4 && kids[n_kids] >= 0) ++n_kids;
+        for (int a = 0; a < 3; ++a) {
+            // the grid spans the padded children exactly: code 0 (value 2) at or below the lowest
+            // plane, code 255 at or above the highest
+            float lo[4], hi[4], glo = INFINITY, ghi = -INFINITY;
+            for (int k = 0; k < n_kids; ++k) {
+                const BNode& c = bnodes[kids[k]];
+                lo[k] = down(c.box.lo[a] - pad);
+                hi[k] = up(c.box.hi[a] + pad);
+                glo = std::min(glo, lo[k]);
+                ghi = std::max(ghi, hi[k]);
+            }
+            const double v0 = plane_value(0), v1 = plane_value(255);
+            float scl = up((float)(((double)ghi - (double)glo) / (v1 - v0)));
+            float org = 0.0f;
+            // (coordinates near the float range's end, beyond what the exact tests can answer, get
+            // the whole grid of a point)
+            const bool ok = std::isfinite(scl) && std::isfinite((float)((double)glo - v0 * (double)scl));
+            if (!ok) scl = 0.0f;
+            while (ok) {
+                org = down((float)((double)glo - v0 * (double)scl));
+                if ((double)org + v1 * (double)scl >= (double)ghi) break;
+                scl = up(scl);
+            }
+            q.org[a] = org;
+            q.scl[a] = scl;
+            uint32_t lw = 0xffffffffu, hw = 0u;
+            for (int k = 0; k < n_kids; ++k) {
+                // the largest code at or below the low plane, the smallest at or above the high one
+                const auto at = [&](int v) { return (double)org + (double)plane_value((uint32_t)v) * (double)scl; };
+                int l = 0, h = 255;
+                if (ok) l = code_of(((double)lo[k] - org) / scl), h = code_of(((double)hi[k] - org) / scl);
+                while (ok && l > 0 && at(l) > (double)lo[k]) --l;
+                while (ok && l < 255 && at(l + 1) <= (double)lo[k]) ++l;
+                while (ok && h < 255 && at(h) < (double)hi[k]) ++h;
+                while (ok && h > 0 && at(h - 1) >= (double)hi[k]) --h;
+                lw = (lw & ~(0xffu << (8 * k))) | ((uint32_t)l << (8 * k));
+                hw |= (uint32_t)h << (8 * k);
+            }
+            q.lo[a] = lw;
+            q.hi[a] = hw;
+        }
     }
 };
 
@@ -339,11 +411,17 @@ int build_qbvh(const float* V, uint64_t nv, const uint32_t* T, uint64_t nt, cons
         mag = std::max(mag, std::fabs(root.lo[a]));
         mag = std::max(mag, std::fabs(root.hi[a]));
     }
-    const float pad = mag * 7.62939453125e-06f;  // 2^-17
+    // 2^-16: covers the roundings of the slab distances (the reciprocal direction to 1 ulp, the
+    // grid's origin relative to the ray's, the planes) for rays from up to about 50 mag away
+    const float pad = mag * 1.52587890625e-05f;
     const double ra = root.area() > 0 ? root.area() : 1.0;
     Collapser col(bnodes, pad, ra, opts.traversal_cost > 0 ? opts.traversal_cost : 1.0);
     col.qnodes.reserve(bnodes.size() / 3 + 1);
+    col.members.reserve(bnodes.size() / 3 + 1);
     col.emit(r, 0, 0);
+    in_pieces(col.qnodes.size(), threads, [&](size_t begin, size_t end) {
+        for (size_t k = begin; k < end; ++k) col.quantise(k);
+    });
 
     out.n_nodes = col.qnodes.size();
     out.nodes = (QNode*)std::aligned_alloc(128, out.n_nodes * sizeof(QNode));
@@ -356,27 +434,29 @@ int build_qbvh(const float* V, uint64_t nv, const uint32_t* T, uint64_t nt, cons
         out.nodes = nullptr;
         return fail(LIAR_ERR_OOM, "host allocation of triangles failed");
     }
-    for (uint64_t k = 0; k < np; ++k) {
-        const uint32_t i = idx[k];
-        QTri& q = out.tris[k];
-        int32_t ii = (int32_t)i;
-        float wbits;
-        std::memcpy(&wbits, &ii, 4);
-        if (i >= nt) {
-            // a sphere: centre and index bits, then the radius with the sphere flag in e1.w
-            const float* sp = S + 4 * (i - nt);
-            q.v0 = {sp[0], sp[1], sp[2], wbits};
-            q.e1 = {sp[3], 0.0f, 0.0f, 1.0f};
-            q.e2 = {0.0f, 0.0f, 0.0f, 0.0f};
-            continue;
+    in_pieces(np, threads, [&](size_t begin, size_t end) {
+        for (size_t k = begin; k < end; ++k) {
+            const uint32_t i = idx[k];
+            QTri& q = out.tris[k];
+            int32_t ii = (int32_t)i;
+            float wbits;
+            std::memcpy(&wbits, &ii, 4);
+            if (i >= nt) {
+                // a sphere: centre and index bits, then the radius with the sphere flag in e1.w
+                const float* sp = S + 4 * (i - nt);
+                q.v0 = {sp[0], sp[1], sp[2], wbits};
+                q.e1 = {sp[3], 0.0f, 0.0f, 1.0f};
+                q.e2 = {0.0f, 0.0f, 0.0f, 0.0f};
+                continue;
+            }
+            const float* a = V + 3 * T[3 * i + 0];
+            const float* bb = V + 3 * T[3 * i + 1];
+            const float* c = V + 3 * T[3 * i + 2];
+            q.v0 = {a[0], a[1], a[2], wbits};
+            q.e1 = {bb[0] - a[0], bb[1] - a[1], bb[2] - a[2], 0.0f};
+            q.e2 = {c[0] - a[0], c[1] - a[1], c[2] - a[2], 0.0f};
         }
-        const float* a = V + 3 * T[3 * i + 0];
-        const float* bb = V + 3 * T[3 * i + 1];
-        const float* c = V + 3 * T[3 * i + 2];
-        q.v0 = {a[0], a[1], a[2], wbits};
-        q.e1 = {bb[0] - a[0], bb[1] - a[1], bb[2] - a[2], 0.0f};
-        q.e2 = {c[0] - a[0], c[1] - a[1], c[2] - a[2], 0.0f};
-    }
+    });
     out.n_leaves = col.leaves;
     out.max_depth = col.max_depth;
     out.stack_needed = col.max_stack;

@@ -42,6 +42,7 @@ constexpr size_t kNoAllocMaxRays = (size_t)1 << 31;
 struct NoAllocDevice {
     uint32_t* scratch = nullptr;  // device address of g_noalloc_scratch on this device
     unsigned blocks[2] = {};      // persistent grid of the closest-hit [0] and any-hit [1] kernel
+    uint32_t sms = 1;
 };
 std::mutex g_setup_mutex;
 NoAllocDevice g_dev[kMaxDevices];
@@ -80,6 +81,7 @@ int noalloc_setup(int device) {
     }
     NoAllocDevice d;
     d.scratch = static_cast<uint32_t*>(ptr);
+    d.sms = (uint32_t)sms;
     int rc = resident_blocks<false>(sms, &d.blocks[0]);
     if (rc == LIAR_OK) rc = resident_blocks<true>(sms, &d.blocks[1]);
     if (rc != LIAR_OK) return rc;
@@ -92,17 +94,16 @@ template <bool ANY>
 int launch_noalloc(const QNode* nodes, const QTri* tris, const liar_ray* rays, uint32_t n, liar_hit* hits,
                    cudaStream_t st, const NoAllocDevice& d) {
     const size_t smem = (size_t)kStackNA * kBlockNA * 8;
-    uint64_t blocks = d.blocks[ANY ? 1 : 0];
-    const uint64_t needed = ((uint64_t)n + kBlockNA - 1) / kBlockNA;
-    if (blocks > needed) blocks = needed;
+    const uint32_t warps = trace_warps(n, d.blocks[ANY ? 1 : 0] * (kBlockNA / 32), d.sms);
+    const uint32_t blocks = (warps + kBlockNA / 32 - 1) / (kBlockNA / 32);
     // the array keeps whatever the previous call left: the counter and the status start at zero
     if (cudaMemsetAsync(d.scratch, 0, 2 * sizeof(uint32_t), st) != cudaSuccess) {
         cudaGetLastError();
         return LIAR_ERR_CUDA;
     }
-    trace_kernel<ANY, kStackNA, kBlockNA, false><<<(unsigned)blocks, kBlockNA, smem, st>>>(
+    trace_kernel<ANY, kStackNA, kBlockNA, false><<<blocks, kBlockNA, smem, st>>>(
         nodes, tris, rays, hits, n, d.scratch, d.scratch + 1, nullptr,
-        trace_batch(n, (uint32_t)blocks * (kBlockNA / 32)), nullptr);
+        trace_batch(n, blocks * (kBlockNA / 32)), nullptr);
     if (cudaGetLastError() != cudaSuccess) return LIAR_ERR_CUDA;
     return LIAR_OK;
 }

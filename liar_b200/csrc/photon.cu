@@ -6,18 +6,17 @@
 // nearest to a point, all closer than r_max, the farthest first in the reference's heap.
 //
 // Build (spatial hashing, Teschner et al. 2003): a bounding-box reduction fixes the grid origin;
-// the cell width follows the photons' density (map_build_impl: about 60 photons per cell on
-// surfaces, 4 in volumes, between r_max and r_max / 8), cell = floor((p - origin) / cell_size),
+// the cell width follows the photons' density (map_build_impl: about 140 photons per cell on
+// surfaces, 9 in volumes, between r_max and r_max / 8), cell = floor((p - origin) / cell_size),
 // bucket = hash(cell) mod 2^m; a counting sort (histogram, exclusive scan, scatter) orders the photons by
 // bucket into float4 (x, y, z, original index) records, each with its packed cell key beside it.
 // Gather: one warp per query visits the cells around the query in rings of growing Chebyshev
-// distance R and stops after ring R as soon as the current k-th distance is at most R cell
-// widths (every photon of a later ring is farther than that), or R cell widths reach r_max --
-// the grid form of the kd-tree search that shrinks its radius as it finds neighbours. Candidates
-// are filtered by their cell key, so buckets shared by colliding cells never yield a photon twice.
-// The k = 64 nearest are a sorted list of 64-bit keys (d^2 bits << 32 | photon index), two per
-// lane; a batch of 32 candidates is sorted by a shuffle bitonic network and merged in with
-// half-cleaners, batches with no key below the current k-th are skipped.
+// distance R until k candidates are found or R cell widths reach r_max, then the cells left of the
+// box around the k-th of them -- the grid form of the kd-tree search that shrinks its radius as it
+// finds neighbours. Candidates are filtered by their cell key, so buckets shared by colliding cells
+// never yield a photon twice. Candidates are 64-bit keys (d^2 bits << 32 | photon index), appended to
+// a list in shared memory while they are below the limit, the list's k-th as of the last cut; the
+// list is sorted once, at the end.
 // Distances use explicitly rounded IEEE operations in a fixed order, so every (query, photon) key
 // and therefore the neighbour set, ties included (equal d^2: lower index first), equals the CPU
 // restatement's.
@@ -317,43 +316,36 @@ __device__ __forceinline__ int div_small(int i, int d, float inv_d) {
     return q;
 }
 
-// cell i of the shell at Chebyshev distance R >= 1 around a cell ((2R+1)^3 - (2R-1)^3 cells): the
+// (div_small's correction step and the cell bound's slack cover the last bits of these)
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// cell i of the shell at Chebyshev distance R >= 2 around a cell ((2R+1)^3 - (2R-1)^3 cells): the
 // two z faces, then the square rings of the levels between them
 __device__ __forceinline__ void shell_cell(int i, int R, int& dx, int& dy, int& dz) {
     const int side = 2 * R + 1, face = side * side;
     if (i < 2 * face) {
         const int j = i < face ? i : i - face;
         dz = i < face ? -R : R;
-        const int y = div_small(j, side, 1.0f / (float)side);
+        const int y = div_small(j, side, rcp_approx((float)side));
         dy = y - R;
         dx = j - y * side - R;
     } else {
         const int per = 8 * R, i2 = i - 2 * face;
-        const int level = div_small(i2, per, 1.0f / (float)per);
+        const int level = div_small(i2, per, rcp_approx((float)per));
         dz = level - R + 1;
         const int p = i2 - level * per;
-        const int k = div_small(p, 2 * R, 1.0f / (float)(2 * R)), t = p - k * 2 * R;
+        const int k = div_small(p, 2 * R, rcp_approx((float)(2 * R))), t = p - k * 2 * R;
         dx = k == 0 ? -R + t : k == 1 ? R : k == 2 ? R - t : -R;
         dy = k == 0 ? -R : k == 1 ? -R + t : k == 2 ? R : R - t;
-    }
-}
-
-// inserts key x into the ascending 64-list (lo: slots 0..31, hi: 32..63, one of each per lane),
-// dropping the largest; every lane takes part (the branches are warp-uniform)
-constexpr int kInsertMax = 8;  // batches with more keys below the k-th take the bitonic merge
-__device__ __forceinline__ void insert_key(uint64_t x, uint64_t& lo, uint64_t& hi) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const int p = __popc(__ballot_sync(0xffffffffu, lo < x));  // lo is ascending: the entries below x lead
-    const uint64_t lo_up = __shfl_up_sync(0xffffffffu, (unsigned long long)lo, 1);
-    const uint64_t lo_last = __shfl_sync(0xffffffffu, (unsigned long long)lo, 31);
-    const uint64_t hi_up = __shfl_up_sync(0xffffffffu, (unsigned long long)hi, 1);
-    if (p < 32) {
-        // x at slot p; lo[31] becomes hi[0]; hi moves up one slot
-        lo = (int)lane < p ? lo : ((int)lane == p ? x : lo_up);
-        hi = lane == 0 ? lo_last : hi_up;
-    } else {
-        const int q = __popc(__ballot_sync(0xffffffffu, hi < x));
-        if (q < 32) hi = (int)lane < q ? hi : ((int)lane == q ? x : hi_up);
     }
 }
 
@@ -366,15 +358,119 @@ struct GatherParams {
     uint32_t n_photons;
 };
 
-__global__ void __launch_bounds__(256) k_gather(const float4* __restrict__ sorted, const uint64_t* __restrict__ cell_key,
+// The nearest candidates of a warp's query, unordered, in shared memory: every candidate whose key is
+// below `limit` is appended; once kCandSpare more than k are held, all but the k nearest (and up to
+// kCandSlack more) are dropped and the limit falls to the farthest kept.
+constexpr int kCandCap = kGatherK + 96, kCandSpare = 64, kCandSlack = 8;
+constexpr int kCandRegs = kCandCap / 32;
+
+// Drops all but the k smallest of the n >= k keys at buf, and up to `slack` more; returns the number
+// kept and in `limit` a key with exactly those below it. The threshold is searched in the
+// distance bits: by interpolation (on surfaces the number of photons grows linearly with d^2), key by
+// key once it is a few short, and by bisection if neither ends it; among equal distances at the
+// threshold, in the index bits.
+__device__ __forceinline__ int keep_nearest(uint64_t* buf, int n, int k, int slack, uint64_t& limit) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint64_t key[kCandRegs];
+    uint32_t top = 0, bottom = 0xffffffffu;
+#pragma unroll
+    for (int r = 0; r < kCandRegs; ++r) {
+        const int j = 32 * r + (int)lane;
+        key[r] = j < n ? buf[j] : ~0ull;
+        bottom = min(bottom, (uint32_t)(key[r] >> 32));
+        if (j < n) top = max(top, (uint32_t)(key[r] >> 32));
+    }
+    uint32_t lo = __reduce_min_sync(0xffffffffu, bottom), hi = __reduce_max_sync(0xffffffffu, top);  // count(<= hi) = n
+    int c_lo = 0, c_hi = n;
+    const auto count = [&](uint32_t d) {
+        int c = 0;
+#pragma unroll
+        for (int r = 0; r < kCandRegs; ++r) c += (uint32_t)(key[r] >> 32) <= d;
+        return __reduce_add_sync(0xffffffffu, c);
+    };
+    // count(lo) = c_lo < k from here on, below the smallest distance or, where that is zero, counted
+    if (lo != 0u) {
+        --lo;
+    } else {
+        c_lo = count(0u);
+        if (c_lo >= k) hi = 0u, c_hi = c_lo;
+    }
+    for (int it = 0; c_hi > k + slack && hi - lo > 1u; ++it) {
+        uint32_t mid = lo + ((hi - lo) >> 1);
+        if (k - c_lo <= 4 && it > 1) {
+            // a few keys short: the next distance above (ties make it more than one key); there is one
+            // up to hi, so that this ends within k - c_lo steps and one more
+            uint32_t next = 0xffffffffu;
+#pragma unroll
+            for (int r = 0; r < kCandRegs; ++r) {
+                const uint32_t d = (uint32_t)(key[r] >> 32);
+                if (d > lo) next = min(next, d);
+            }
+            mid = min(__reduce_min_sync(0xffffffffu, next), hi - 1u);
+        } else if (it < 8) {
+            const float f = ((float)(k - c_lo) + 0.5f * (float)slack) * rcp_approx((float)(c_hi - c_lo));
+            const float a = __uint_as_float(lo), b = __uint_as_float(hi);
+            mid = min(max(__float_as_uint(fmaf(b - a, f, a)), lo + 1u), hi - 1u);
+        }
+        const int c = count(mid);
+        if (c >= k) {
+            hi = mid;
+            c_hi = c;
+        } else {
+            lo = mid;
+            c_lo = c;
+        }
+    }
+    uint32_t low = 0xffffffffu;  // the threshold's index bits
+    if (c_hi > k + slack) {
+        // more than that at one distance: the lowest indices of them
+        uint32_t i_lo = 0, i_hi = 0xffffffffu;  // count(<= (hi, i_hi)) = c_hi
+        const auto count_low = [&](uint32_t i) {
+            const uint64_t t = ((uint64_t)hi << 32) | i;
+            int c = 0;
+#pragma unroll
+            for (int r = 0; r < kCandRegs; ++r) c += key[r] <= t;
+            return __reduce_add_sync(0xffffffffu, c);
+        };
+        if (count_low(0u) >= k) i_hi = 0u;
+        while (i_hi - i_lo > 1u && i_hi != 0u) {
+            const uint32_t mid = i_lo + ((i_hi - i_lo) >> 1);
+            if (count_low(mid) >= k) i_hi = mid;
+            else i_lo = mid;
+        }
+        low = i_hi;
+    }
+    const uint64_t last = ((uint64_t)hi << 32) | low;
+    limit = last + 1ull;
+    int kept = 0;
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < kCandRegs; ++r) {
+        const bool keep = key[r] <= last && 32 * r + (int)lane < n;
+        const uint32_t m = __ballot_sync(0xffffffffu, keep);
+        if (keep) buf[kept + __popc(m & ((1u << lane) - 1u))] = key[r];
+        kept += __popc(m);
+    }
+    __syncwarp();
+    return kept;
+}
+
+// One warp per query. Bound by issue slots (73% of them, with the candidates' distances a small part):
+// merging every batch of 32 candidates into a sorted list took 3,900 warp instructions a query on 4M
+// photons on surfaces (1M queries, k = 64: 4.96 ms). Here candidates are only filtered by distance and
+// appended, the list is cut to the k nearest two or three times, and sorted once, at the end (2.6 ms,
+// with about seven batches of 32 candidates a query).
+__global__ void __launch_bounds__(256, 4) k_gather(const float4* __restrict__ sorted, const uint64_t* __restrict__ cell_key,
                                                 const uint32_t* __restrict__ start, GatherParams G,
                                                 const float* __restrict__ queries, uint32_t nq, int k_out,
                                                 int32_t* __restrict__ out_idx, float* __restrict__ out_d2,
                                                 int32_t* __restrict__ out_count, uint32_t* __restrict__ status,
                                                 const float4* __restrict__ ordered) {
-    const uint32_t lane = threadIdx.x & 31u;
+    __shared__ uint64_t s_cand[8][kCandCap];
+    const uint32_t lane = threadIdx.x & 31u, lt_mask = (1u << lane) - 1u;
     const uint32_t warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
+    uint64_t* cand = s_cand[threadIdx.x >> 5];
     constexpr uint64_t INF = ~0ull;
     const BuildParams& P = G.B;
     for (uint32_t w = warp_global; w < nq; w += n_warps) {
@@ -397,157 +493,201 @@ __global__ void __launch_bounds__(256) k_gather(const float4* __restrict__ sorte
             qz = queries[3 * q + 2];
         }
         const int cx = cell_coord(qx, P.ox, P.inv), cy = cell_coord(qy, P.oy, P.inv), cz = cell_coord(qz, P.oz, P.inv);
-        // the k nearest so far, ascending: slot `lane` in lo, slot `32 + lane` in hi
-        uint64_t lo = INF, hi = INF;
-        uint64_t kth = INF;  // key of the current k-th (64th) nearest
-        for (int R = 0; R <= G.max_ring; ++R) {
-            // the cells at Chebyshev distance R, 32 at a time (lane: one cell)
-            const int shell = R == 0 ? 1 : (2 * R + 1) * (2 * R + 1) * (2 * R + 1) - (2 * R - 1) * (2 * R - 1) * (2 * R - 1);
+        int n = 0;            // candidates held
+        int at_limit = 0;     // candidates held when the limit was last set, 0 while it is that of r_max
+        uint64_t limit = (uint64_t)__float_as_uint(G.r2max) << 32;
+        // rings of cells at Chebyshev distance R, the query's own cell with R = 1, until k candidates are
+        // found; then the cells of the box around their limit that the rings have not covered
+        bool box = false;
+        int bx0 = 0, by0 = 0, bz0 = 0, bnx = 0, bny = 0;  // the box's first cell (relative) and sizes
+        float bix = 0.0f, biy = 0.0f;                     // 1 / (bnx bny), 1 / bnx
+        int R = 1, shell = 27;
+        while (true) {
+            // 32 cells at a time (lane: one cell)
             for (int c0 = 0; c0 < shell; c0 += 32) {
                 const int c = c0 + (int)lane;
                 int dx = 0, dy = 0, dz = 0;
                 bool mine = c < shell;
-                if (mine && R > 0) shell_cell(c, R, dx, dy, dz);
-                int ix = cx + dx, iy = cy + dy, iz = cz + dz;
-                mine = mine && ix >= 0 && iy >= 0 && iz >= 0 && ix <= kCellLimit && iy <= kCellLimit && iz <= kCellLimit;
-                float cell_d2 = 0.0f;  // after the sort: lane j's cell's distance bound (ascending in j)
-                if (R > 0) {
-                    // the query's distance to the cell's box, less the cell-assignment round-off: a
-                    // cell farther than the current k-th (or r_max) cannot contribute and is skipped;
-                    // the others are taken nearest first, so that the k-th falls early and later
-                    // candidates fail the batch test instead of entering the list
-                    float md2 = 0.0f;
-                    if (mine) {
-                        const float bx = P.ox + (float)ix * G.cell, by = P.oy + (float)iy * G.cell, bz = P.oz + (float)iz * G.cell;
-                        const float ex = fmaxf(fmaxf(bx - qx, qx - (bx + G.cell)), 0.0f);
-                        const float ey = fmaxf(fmaxf(by - qy, qy - (by + G.cell)), 0.0f);
-                        const float ez = fmaxf(fmaxf(bz - qz, qz - (bz + G.cell)), 0.0f);
-                        const float md = fmaxf(sqrtf(ex * ex + ey * ey + ez * ez) - G.slack, 0.0f);
-                        md2 = md * md;
-                        const float bound = kth != INF ? fminf(__uint_as_float((uint32_t)(kth >> 32)), G.r2max) : G.r2max;
-                        mine = md2 <= bound;
-                    }
-                    const uint32_t live = __ballot_sync(0xffffffffu, mine);
-                    if (live == 0u) continue;  // nothing in this chunk can come within the k-th
-                    if (live & (live - 1u)) {
-                        // 32-bit sort keys: the bound with its 5 low bits cleared (a lower bound
-                        // still, so that the order stays ascending in the bound the batches test)
-                        // and the lane in those bits
-                        const uint32_t ck = warp_sort32u(mine ? ((__float_as_uint(md2) & ~31u) | lane) : 0xffffffffu);
-                        const int src = (int)(ck & 31u);
-                        mine = ck != 0xffffffffu;
-                        cell_d2 = __uint_as_float(ck & ~31u);
-                        ix = __shfl_sync(0xffffffffu, ix, src);
-                        iy = __shfl_sync(0xffffffffu, iy, src);
-                        iz = __shfl_sync(0xffffffffu, iz, src);
-                    } else {
-                        // one cell: lane 0 takes it
-                        const int src = __ffs(live) - 1;
-                        cell_d2 = __uint_as_float(__float_as_uint(__shfl_sync(0xffffffffu, md2, src)) & ~31u);
-                        ix = __shfl_sync(0xffffffffu, ix, src);
-                        iy = __shfl_sync(0xffffffffu, iy, src);
-                        iz = __shfl_sync(0xffffffffu, iz, src);
-                        mine = lane == 0;
-                    }
+                if (box) {
+                    dz = div_small(c, bnx * bny, bix);
+                    const int l = c - dz * bnx * bny;
+                    dy = div_small(l, bnx, biy);
+                    dx = l - dy * bnx + bx0;
+                    dy += by0;
+                    dz += bz0;
+                    mine = mine && max(abs(dx), max(abs(dy), abs(dz))) > R;
+                } else if (R == 1) {
+                    dz = (int)(lane * 57u >> 9) - 1;  // lane / 9
+                    const uint32_t l9 = lane - 9u * (uint32_t)(dz + 1);
+                    dy = (int)(l9 * 11u >> 5) - 1;  // l9 / 3
+                    dx = (int)l9 - 3 * (dy + 1) - 1;
+                } else if (mine) {
+                    shell_cell(c, R, dx, dy, dz);
                 }
-                uint32_t s0 = 0, s1 = 0;
-                uint64_t my_key = pack_cell(ix, iy, iz);
+                const int ix = cx + dx, iy = cy + dy, iz = cz + dz;
+                mine = mine && ix >= 0 && iy >= 0 && iz >= 0 && ix <= kCellLimit && iy <= kCellLimit && iz <= kCellLimit;
+                float md2 = 0.0f;
+                if (mine) {
+                    // the query's distance to the cell's box, less the cell-assignment round-off: a
+                    // cell beyond the limit cannot contribute and is skipped; the others are taken
+                    // nearest first, so that the limit falls early
+                    const float lx = P.ox + (float)ix * G.cell, ly = P.oy + (float)iy * G.cell, lz = P.oz + (float)iz * G.cell;
+                    const float ex = fmaxf(fmaxf(lx - qx, qx - (lx + G.cell)), 0.0f);
+                    const float ey = fmaxf(fmaxf(ly - qy, qy - (ly + G.cell)), 0.0f);
+                    const float ez = fmaxf(fmaxf(lz - qz, qz - (lz + G.cell)), 0.0f);
+                    const float md = fmaxf(sqrt_approx(ex * ex + ey * ey + ez * ez) * 0.999999f - G.slack, 0.0f);
+                    md2 = md * md;
+                    mine = md2 <= __uint_as_float((uint32_t)(limit >> 32));
+                }
+                uint32_t s0 = 0, cnt = 0;
+                bool mixed = false;
+                const uint64_t my_key = pack_cell(ix, iy, iz);
                 if (mine) {
                     const uint32_t b = bucket_of(ix, iy, iz, P.mask);
                     const uint32_t r0 = __ldg(start + b);
                     s0 = r0 & ~kBucketMixed;
-                    s1 = __ldg(start + b + 1) & ~kBucketMixed;
+                    const uint32_t s1 = __ldg(start + b + 1) & ~kBucketMixed;
                     if (s0 > s1 || s1 > G.n_photons) {  // corrupt bucket range: record it, skip the cell
                         atomicOr(status, kStatusBadBucket);
-                        s0 = s1 = 0;
-                    }
-                    if (s1 > s0 && !(r0 & kBucketMixed)) {
+                    } else {
+                        cnt = s1 - s0;
+                        mixed = (r0 & kBucketMixed) != 0u;
                         // a single-cell bucket: its first key tells whether it is this cell's
-                        if (__ldg(reinterpret_cast<const unsigned long long*>(cell_key) + s0) != my_key) s1 = s0;
-                        else my_key |= 1ull << 63;  // every photon of the range belongs to the cell
+                        if (cnt && !mixed && __ldg(reinterpret_cast<const unsigned long long*>(cell_key) + s0) != my_key) cnt = 0;
                     }
                 }
-                // the chunk's photons as one list: lane j's cell owns items [excl_j, excl_j + cnt_j)
-                // of it, so that a batch of 32 candidates spans as many cells as it takes (cells
-                // hold a photon or two on average; one batch per cell would leave most lanes idle)
-                // (64-bit counts: 32 colliding cells of one huge bucket must not wrap)
-                const uint64_t cnt = s1 - s0;
-                uint64_t incl = cnt;
+                uint32_t live = __ballot_sync(0xffffffffu, cnt > 0u);
+                if (live == 0u) continue;
+                uint32_t n_live = __popc(live);
+                // mixed buckets are taken one by one, with the cell's key checked photon by photon (and
+                // so are, for the 32-bit prefix sums, buckets of 2^27 photons)
+                const uint32_t slow = __ballot_sync(0xffffffffu, mixed && cnt > 0u) | __ballot_sync(0xffffffffu, cnt >> 27);
+                while (live) {
+                    const bool check = (live & ~slow) == 0u;
+                    const uint32_t take = check ? live & (0u - live) : live & ~slow;
+                    live &= ~take;
+                    // the cells taken, nearest first, in lanes 0 .. n_live - 1: sorted by the distance
+                    // bound with its 5 low bits cleared (a lower bound still) and the lane in them
+                    n_live = __popc(take);
+                    const uint32_t ck = n_live == 1u ? (uint32_t)__ffs(take) - 1u
+                                                     : warp_sort32u((take >> lane) & 1u ? ((__float_as_uint(md2) & ~31u) | lane) : 0xffffffffu);
+                    const int src = (int)(ck & 31u);
+                    const float a_d2 = __uint_as_float(ck & ~31u);
+                    const uint32_t a_s0 = __shfl_sync(0xffffffffu, s0, src), c_src = __shfl_sync(0xffffffffu, cnt, src);
+                    const uint32_t a_cnt = lane < n_live ? c_src : 0u;
+                    const uint64_t target = check ? __shfl_sync(0xffffffffu, (unsigned long long)my_key, src) : 0ull;
+                    // their photons as one list: lane j's cell owns items [excl_j, excl_j + cnt_j), so
+                    // that a batch of 32 candidates spans as many cells as it takes
+                    uint32_t incl = a_cnt;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint64_t t = __shfl_up_sync(0xffffffffu, (unsigned long long)incl, o);
-                    if ((int)lane >= o) incl += t;
-                }
-                const uint64_t total = __shfl_sync(0xffffffffu, (unsigned long long)incl, 31);
-                const uint64_t excl = incl - cnt;
-                for (uint64_t base = 0; base < total; base += 32) {
-                    const uint64_t item = base + lane;
-                    // the owning cell: the last lane whose list starts at or before the item
-                    // (every lane runs the same shuffles)
-                    uint32_t owner = 0;
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+                        if ((int)lane >= o) incl += t;
+                    }
+                    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31), excl = incl - a_cnt, from = a_s0 - excl;
+                    for (uint32_t base = 0; base < total; base += 32) {
+                        const uint32_t item = base + lane;
+                        // the owning cell: the last lane whose list starts at or before the item
+                        uint32_t owner = 0;
+                        if (n_live > 1u) {
 #pragma unroll
-                    for (uint32_t step = 16; step > 0; step >>= 1) {
-                        const uint64_t e = __shfl_sync(0xffffffffu, (unsigned long long)excl, (int)(owner + step));
-                        if (e <= item) owner += step;
-                    }
-                    // the cells are in ascending distance order: once the batch's first cell lies
-                    // beyond the current k-th, so do all that follow
-                    if (R > 0 && kth != INF) {
-                        const float first_d2 = __shfl_sync(0xffffffffu, cell_d2, (int)__shfl_sync(0xffffffffu, owner, 0));
-                        if (first_d2 > __uint_as_float((uint32_t)(kth >> 32))) break;
-                    }
-                    const uint32_t o_s0 = __shfl_sync(0xffffffffu, s0, (int)owner);
-                    const uint64_t o_excl = __shfl_sync(0xffffffffu, (unsigned long long)excl, (int)owner);
-                    const uint64_t target = __shfl_sync(0xffffffffu, (unsigned long long)my_key, (int)owner);
-                    uint64_t key = INF;
-                    if (item < total) {
-                        const uint32_t i = o_s0 + (uint32_t)(item - o_excl);
-                        const float4 p = __ldg(sorted + i);
-                        const bool in_cell = (target >> 63) != 0ull ||
-                                             __ldg(reinterpret_cast<const unsigned long long*>(cell_key) + i) == target;
-                        if (in_cell) {
+                            for (uint32_t step = 16; step > 0; step >>= 1) {
+                                const uint32_t e = __shfl_sync(0xffffffffu, excl, (int)(owner + step));
+                                if (e <= item && owner + step < n_live) owner += step;
+                            }
+                            // ascending distances: once the batch's first cell lies beyond the limit,
+                            // so do all that follow
+                            const float first = __shfl_sync(0xffffffffu, a_d2, (int)__shfl_sync(0xffffffffu, owner, 0));
+                            if (first > __uint_as_float((uint32_t)(limit >> 32))) break;
+                        }
+                        const uint32_t i = __shfl_sync(0xffffffffu, from, (int)owner) + item;
+                        uint64_t key = INF;
+                        if (item < total) {
+                            const float4 p = __ldg(sorted + i);
                             const float d2 = dist2_exact(p.x, p.y, p.z, qx, qy, qz);
-                            if (d2 < G.r2max) key = ((uint64_t)__float_as_uint(d2) << 32) | (uint64_t)__float_as_uint(p.w);
+                            key = ((uint64_t)__float_as_uint(d2) << 32) | (uint64_t)__float_as_uint(p.w);
+                            if (check && __ldg(reinterpret_cast<const unsigned long long*>(cell_key) + i) != target) key = INF;
+                        }
+                        const bool better = key < limit;
+                        const uint32_t m = __ballot_sync(0xffffffffu, better);
+                        if (m == 0u) continue;
+                        if (better) cand[n + __popc(m & lt_mask)] = key;
+                        n += __popc(m);
+                        if (n >= k_out + kCandSpare) {
+                            __syncwarp();
+                            at_limit = n = keep_nearest(cand, n, k_out, kCandSlack, limit);
                         }
                     }
-                    const uint32_t better = __ballot_sync(0xffffffffu, key < kth);
-                    if (better == 0u) continue;
-                    if (__popc(better) <= kInsertMax) {
-                        // a few keys below the k-th: insert them one at a time
-                        uint32_t m = better;
-                        while (m) {
-                            const int src = __ffs(m) - 1;
-                            m &= m - 1;
-                            insert_key(__shfl_sync(0xffffffffu, (unsigned long long)key, src), lo, hi);
-                        }
-                        kth = __shfl_sync(0xffffffffu, (unsigned long long)hi, 31);
-                        continue;
-                    }
-                    const uint64_t bsort = warp_sort32(key);
-                    // smallest 32 of hi and the batch: half-cleaner against the reversed batch
-                    // (every shuffle is executed by all 32 lanes, outside lane-dependent branches)
-                    const uint64_t brev = reverse_lanes(bsort);
-                    uint64_t m = hi < brev ? hi : brev;
-                    m = warp_bitonic_merge32(m);
-                    // lo (sorted) and m (sorted): split into the lower and upper 32
-                    const uint64_t mr = reverse_lanes(m);
-                    const uint64_t nlo = lo < mr ? lo : mr;
-                    const uint64_t nhi = lo < mr ? mr : lo;
-                    lo = warp_bitonic_merge32(nlo);
-                    hi = warp_bitonic_merge32(nhi);
-                    kth = __shfl_sync(0xffffffffu, (unsigned long long)hi, 31);
                 }
             }
+            if (box) break;
             // every photon outside rings 0..R is farther than R cells (minus round-off)
             const float reach = fmaxf((float)R * G.cell - G.slack, 0.0f);
-            const uint64_t kk = __shfl_sync(0xffffffffu, (unsigned long long)(k_out > 32 ? hi : lo), (k_out - 1) & 31);
-            if (kk != INF && __uint_as_float((uint32_t)(kk >> 32)) <= reach * reach) break;
             if (reach * reach >= G.r2max) break;
+            if (n >= k_out && n != at_limit) {
+                __syncwarp();
+                at_limit = n = keep_nearest(cand, n, k_out, kCandSlack, limit);
+            }
+            if (at_limit) {
+                // the cells that a photon below the limit can lie in
+                const float rho = sqrt_approx(__uint_as_float((uint32_t)(limit >> 32))) * 1.000001f + G.slack;
+                bx0 = cell_coord(qx - rho, P.ox, P.inv) - cx;
+                by0 = cell_coord(qy - rho, P.oy, P.inv) - cy;
+                bz0 = cell_coord(qz - rho, P.oz, P.inv) - cz;
+                const int bx1 = cell_coord(qx + rho, P.ox, P.inv) - cx, by1 = cell_coord(qy + rho, P.oy, P.inv) - cy,
+                          bz1 = cell_coord(qz + rho, P.oz, P.inv) - cz;
+                if (min(bx0, min(by0, bz0)) >= -R && max(bx1, max(by1, bz1)) <= R) break;
+                box = true;
+                bnx = bx1 - bx0 + 1;
+                bny = by1 - by0 + 1;
+                shell = bnx * bny * (bz1 - bz0 + 1);
+                bix = rcp_approx((float)(bnx * bny));
+                biy = rcp_approx((float)bnx);
+                continue;
+            }
+            if (++R > G.max_ring) break;
+            shell = (2 * R + 1) * (2 * R + 1) * (2 * R + 1) - (2 * R - 1) * (2 * R - 1) * (2 * R - 1);
         }
-        // write the first k_out entries (k_out <= 64) in ascending order
-        const uint32_t cnt_lo = __popc(__ballot_sync(0xffffffffu, lo != INF));
-        const uint32_t cnt_hi = __popc(__ballot_sync(0xffffffffu, hi != INF));
-        const int count = min((int)(cnt_lo + cnt_hi), k_out);
+        __syncwarp();
+        if (n > k_out) n = keep_nearest(cand, n, k_out, 0, limit);
+        // the nearest k in ascending order: slot `lane` in lo, slot `32 + lane` in hi. Sorted by 32-bit
+        // keys, the distance in 2^26 steps of the limit with the place in cand: exchanges of one
+        // shuffle and one minimum; where two distances share a step the order shows it (about one
+        // query in 30,000), and the full keys are sorted
+        const float step = 67108864.0f / __uint_as_float((uint32_t)(limit >> 32));
+        const auto short_key = [&](uint32_t j) {
+            if ((int)j >= n) return 0xffffffffu;
+            const float d2 = __uint_as_float((uint32_t)(cand[j] >> 32));
+            return (min((uint32_t)(d2 * step), 67108862u) << 6) | j;  // below the empty key
+        };
+        uint32_t s_lo = warp_sort32u(short_key(lane)), s_hi = 0xffffffffu;
+        if (n > 32) {
+            s_hi = warp_sort32u(short_key(32u + lane));
+            const uint32_t r_hi = __shfl_sync(0xffffffffu, s_hi, 31 - (int)lane);
+            s_hi = max(s_lo, r_hi);
+            s_lo = min(s_lo, r_hi);
+#pragma unroll
+            for (int j = 16; j > 0; j >>= 1) {
+                const uint32_t a = __shfl_xor_sync(0xffffffffu, s_lo, j), b = __shfl_xor_sync(0xffffffffu, s_hi, j);
+                const bool lower = (lane & (uint32_t)j) == 0u;
+                s_lo = lower ? min(s_lo, a) : max(s_lo, a);
+                s_hi = lower ? min(s_hi, b) : max(s_hi, b);
+            }
+        }
+        uint64_t lo = s_lo != 0xffffffffu ? cand[s_lo & 63u] : INF, hi = s_hi != 0xffffffffu ? cand[s_hi & 63u] : INF;
+        const uint64_t lo_next = __shfl_down_sync(0xffffffffu, (unsigned long long)lo, 1),
+                       hi_next = __shfl_down_sync(0xffffffffu, (unsigned long long)hi, 1),
+                       hi_first = __shfl_sync(0xffffffffu, (unsigned long long)hi, 0);
+        if (__any_sync(0xffffffffu, lo > (lane == 31u ? hi_first : lo_next) || (lane < 31u && hi > hi_next))) {
+            lo = (int)lane < n ? cand[lane] : INF;
+            hi = (int)(32 + lane) < n ? cand[32 + lane] : INF;
+            lo = warp_sort32(lo);
+            hi = reverse_lanes(warp_sort32(hi));
+            const uint64_t a = lo < hi ? lo : hi, b = lo < hi ? hi : lo;
+            lo = warp_bitonic_merge32(a);
+            hi = warp_bitonic_merge32(b);
+        }
+        __syncwarp();
         int32_t* oi = out_idx + (size_t)q * k_out;
         float* od = out_d2 + (size_t)q * k_out;
         if ((int)lane < k_out) {
@@ -558,43 +698,72 @@ __global__ void __launch_bounds__(256) k_gather(const float4* __restrict__ sorte
             oi[32 + lane] = hi != INF ? (int32_t)(uint32_t)hi : -1;
             od[32 + lane] = hi != INF ? __uint_as_float((uint32_t)(hi >> 32)) : INFINITY;
         }
-        if (lane == 0 && out_count) out_count[q] = count;
+        if (lane == 0 && out_count) out_count[q] = min(n, k_out);
     }
 }
 
 // PhotonMapper::estimateIrradianceImpl (photon_mapper.cpp:1254-1279): sum of the powers of the
 // neighbours arriving from the normal's side, over pi r^2 with r the farthest neighbour's distance
-__global__ void k_estimate(const float* __restrict__ power, const float* __restrict__ omega_in,
-                           const float* __restrict__ normals, uint32_t nq, int k, const int32_t* __restrict__ idx,
-                           const float* __restrict__ d2, const int32_t* __restrict__ count, float power_scale,
-                           uint32_t n_photons, float* __restrict__ out, uint32_t* __restrict__ status) {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+//
+// W lanes per query, a neighbour to a lane (two at k > 32). Bound by L1 wavefronts and, with a thread
+// per query (303,000 queries in flight, their photons spread over more than the L2), by DRAM: 5.5 GB
+// read for 96 MB of photons. Lanes share a query, so that the queries in flight are fewer and their
+// neighbours, which overlap, are found in L1 and L2; and a 12-byte record is read as the one or two
+// aligned 16-byte words that hold it.
+__device__ __forceinline__ float3 load_record(const float* __restrict__ p, uint32_t i, uint32_t n, bool aligned) {
+    if (!aligned || i + 2u > n) return make_float3(__ldg(p + 3 * (size_t)i), __ldg(p + 3 * (size_t)i + 1), __ldg(p + 3 * (size_t)i + 2));
+    const uint32_t m = i & 3u;  // the record starts m * 12 bytes after a 48-byte boundary
+    const float4* v = reinterpret_cast<const float4*>(p + 12 * (size_t)(i >> 2)) + (m == 0u ? 0u : m - 1u);
+    const float4 a = __ldg(v);
+    float4 b = a;
+    if (m == 1u || m == 2u) b = __ldg(v + 1);
+    return make_float3(m == 0u ? a.x : m == 1u ? a.w : m == 2u ? a.z : a.y, m == 0u ? a.y : m == 1u ? b.x : m == 2u ? a.w : a.z,
+                       m == 0u ? a.z : m == 1u ? b.y : m == 2u ? b.x : a.w);
+}
+
+template <int W>
+__global__ void __launch_bounds__(256) k_estimate(const float* __restrict__ power, const float* __restrict__ omega_in,
+                                                  const float* __restrict__ normals, uint32_t nq, int k,
+                                                  const int32_t* __restrict__ idx, const float* __restrict__ d2,
+                                                  const int32_t* __restrict__ count, float power_scale, uint32_t n_photons,
+                                                  float* __restrict__ out, uint32_t* __restrict__ status) {
+    const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) / W, sub = threadIdx.x % W;
     if (q >= nq) return;
+    const bool al_p = ((uintptr_t)power & 15u) == 0u, al_o = ((uintptr_t)omega_in & 15u) == 0u;
     const int c = count[q];
     float x = 0.0f, y = 0.0f, z = 0.0f;
-    if (c > 0) {
-        const float nx = normals[3 * q], ny = normals[3 * q + 1], nz = normals[3 * q + 2];
-        for (int j = 0; j < c && j < k; ++j) {
-            const int32_t i = idx[(size_t)q * k + j];
-            if (i < 0 || (uint32_t)i >= n_photons) {
-                atomicOr(status, kStatusBadBucket);
-                continue;
-            }
-            if (omega_in[3 * i] * nx + omega_in[3 * i + 1] * ny + omega_in[3 * i + 2] * nz > 0.0f) {
-                x += power[3 * i];
-                y += power[3 * i + 1];
-                z += power[3 * i + 2];
-            }
+    const float nx = normals[3 * (size_t)q], ny = normals[3 * (size_t)q + 1], nz = normals[3 * (size_t)q + 2];
+    for (int j = (int)sub; j < c && j < k; j += W) {
+        const int32_t i = idx[(size_t)q * k + j];
+        if (i < 0 || (uint32_t)i >= n_photons) {
+            atomicOr(status, kStatusBadBucket);
+            continue;
         }
-        const float r2 = d2[(size_t)q * k + (c < k ? c : k) - 1];
-        const float s = r2 > 0.0f ? power_scale / (3.14159265358979323846f * r2) : 0.0f;
-        x *= s;
-        y *= s;
-        z *= s;
+        const float3 o = load_record(omega_in, (uint32_t)i, n_photons, al_o);
+        if (o.x * nx + o.y * ny + o.z * nz > 0.0f) {
+            const float3 p = load_record(power, (uint32_t)i, n_photons, al_p);
+            x += p.x;
+            y += p.y;
+            z += p.z;
+        }
     }
-    out[3 * q] = x;
-    out[3 * q + 1] = y;
-    out[3 * q + 2] = z;
+    const uint32_t group = W == 32 ? 0xffffffffu : ((1u << (W & 31)) - 1u) << ((threadIdx.x & 31u) / W * W);
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) {
+        x += __shfl_xor_sync(group, x, o);
+        y += __shfl_xor_sync(group, y, o);
+        z += __shfl_xor_sync(group, z, o);
+    }
+    if (sub == 0) {
+        float s = 0.0f;
+        if (c > 0) {
+            const float r2 = d2[(size_t)q * k + (c < k ? c : k) - 1];
+            s = r2 > 0.0f ? power_scale / (3.14159265358979323846f * r2) : 0.0f;
+        }
+        out[3 * (size_t)q] = x * s;
+        out[3 * (size_t)q + 1] = y * s;
+        out[3 * (size_t)q + 2] = z * s;
+    }
 }
 
 int map_build_impl(liar_gpu_ctx* ctx, liar_gpu_photon_map* m, const float* d_pos, size_t n, cudaStream_t st) {
@@ -685,10 +854,12 @@ int map_build_impl(liar_gpu_ctx* ctx, liar_gpu_photon_map* m, const float* d_pos
         // sharing a photon's cell, lambda(c) (a bucket's count squared summed over the buckets, over
         // n, less the photon itself and the expected share of colliding cells n / nb), at r_max / 2
         // and r_max / 4 gives the local dimension D = log2(lambda1 / lambda2) (2 for photons on
-        // surfaces, 3 in volumes) and the width at which lambda = T(D), 60 on surfaces and 4 in
-        // volumes (geometric in between), measured optima of the ring walk's cost: the bucket
-        // lookups of the cells visited (queries with fewer than k photons within r_max visit all
-        // of them) against the candidates tested; cells r_max / 1 .. r_max / 8
+        // surfaces, 3 in volumes) and the width at which lambda = T(D), 140 on surfaces and 9 in
+        // volumes (geometric in between), measured optima of the gather's cost: the bucket lookups of
+        // the cells visited against the candidates tested. Rebuild, gather and estimate at (60, 4),
+        // (120, 8), (180, 12), (240, 16): 4M photons on surfaces, 1M queries, k = 64: 4.98, 4.12,
+        // 4.02, 4.18 ms; 1M photons in a volume, 500k queries, k = 32: 1.93, 1.62, 1.58, 1.61 ms;
+        // 50k photons, 3,000 queries, k = 50: 156, 169, 178, 186 us; cells r_max / 1 .. r_max / 8
         if (n >= 1024) {
             double lam[2] = {0.0, 0.0};
             unsigned long long* d_sum = reinterpret_cast<unsigned long long*>(bounds + 8);
@@ -709,7 +880,7 @@ int map_build_impl(liar_gpu_ctx* ctx, liar_gpu_photon_map* m, const float* d_pos
             float refine = kRefine;
             if (lam[0] > 0.0 && lam[1] > 0.0) {
                 const double D = std::min(3.0, std::max(1.5, std::log2(lam[0] / lam[1])));
-                const double target = 60.0 * std::pow(4.0 / 60.0, D - 2.0);
+                const double target = 140.0 * std::pow(9.0 / 140.0, D - 2.0);
                 refine = (float)std::min(8.0, std::max(1.0, 2.0 * std::pow(lam[0] / target, 1.0 / D)));
             }
             while (!set_grid(m->r_max / refine) && refine > 1.0f) refine = std::max(1.0f, refine * 0.5f);
@@ -979,9 +1150,15 @@ extern "C" int liar_gpu_photon_estimate_device(liar_gpu_ctx* ctx, const float* d
     int rc = ctx_activate(ctx);
     if (rc) return rc;
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-    k_estimate<<<(unsigned)((n_queries + 255) / 256), 256, 0, st>>>(d_power, d_omega_in, d_normals, (uint32_t)n_queries, k,
-                                                                   d_idx, d_d2, d_count, power_scale,
-                                                                   (uint32_t)n_photons, d_out,
-                                                                   ctx->d_scratch + kStatusWord);
+    // lanes per query: k of them up to a warp (fewer queries in flight at once read photons nearer to
+    // one another, see k_estimate)
+    const auto launch = [&](auto kern, int w) {
+        kern<<<(unsigned)((n_queries * (size_t)w + 255) / 256), 256, 0, st>>>(
+            d_power, d_omega_in, d_normals, (uint32_t)n_queries, k, d_idx, d_d2, d_count, power_scale, (uint32_t)n_photons,
+            d_out, ctx->d_scratch + kStatusWord);
+    };
+    if (k <= 8) launch(k_estimate<8>, 8);
+    else if (k <= 16) launch(k_estimate<16>, 16);
+    else launch(k_estimate<32>, 32);
     return ctx_cuda(ctx, cudaGetLastError(), "photon estimate launch");
 }

@@ -9,7 +9,7 @@
 // the cell width follows the photons' density (map_build_impl: about 140 photons per cell on
 // surfaces, 9 in volumes, between r_max and r_max / 8), cell = floor((p - origin) / cell_size),
 // bucket = hash(cell) mod 2^m; a counting sort (histogram, exclusive scan, scatter) orders the photons by
-// bucket into float4 (x, y, z, original index) records, each with its packed cell key beside it.
+// bucket into float4 (x, y, z, original index) records (their cells follow from the positions).
 // Gather: one warp per query visits the cells around the query in rings of growing Chebyshev
 // distance R until k candidates are found or R cell widths reach r_max, then the cells left of the
 // box around the k-th of them -- the grid form of the kd-tree search that shrinks its radius as it
@@ -41,27 +41,22 @@ struct liar_gpu_photon_map {
     float extent = 0.0f;
     uint32_t bucket_bits = 0;
     float4* sorted = nullptr;          // bucket order: x, y, z, original index bits
-    uint64_t* cell_key = nullptr;      // packed cell of each sorted photon
     uint32_t* bucket_start = nullptr;  // 2^bits + 1
-    void* scratch = nullptr;           // build scratch (bucket keys, counts, bounds), kept for rebuilds
+    void* scratch = nullptr;           // build scratch (ranks, counts, bounds), kept for rebuilds
     size_t scratch_bytes = 0;
-    size_t cap_n = 0, cap_buckets = 0; // capacities of sorted / cell_key and of bucket_start
+    size_t cap_n = 0, cap_buckets = 0; // capacities of sorted and of bucket_start
 };
 
 namespace {
 
 constexpr int kGatherK = 64;
 constexpr float kRefine = 4.0f;              // cells per r_max
-constexpr int kCellBits = 21;                // per axis in the packed cell key
-constexpr int kCellLimit = (1 << kCellBits) - 2;
+constexpr int kCellLimit = (1 << 21) - 2;     // largest cell index per axis
 constexpr uint32_t kStatusBadBucket = 1u << 4;  // device status bit of the photon kernels
 
 __host__ __device__ __forceinline__ uint32_t bucket_of(int ix, int iy, int iz, uint32_t mask) {
     const uint32_t h = ((uint32_t)ix * 73856093u) ^ ((uint32_t)iy * 19349663u) ^ ((uint32_t)iz * 83492791u);
     return h & mask;
-}
-__host__ __device__ __forceinline__ uint64_t pack_cell(int ix, int iy, int iz) {
-    return ((uint64_t)(uint32_t)ix << (2 * kCellBits)) | ((uint64_t)(uint32_t)iy << kCellBits) | (uint64_t)(uint32_t)iz;
 }
 __device__ __forceinline__ int cell_coord(float p, float o, float inv) { return (int)floorf((p - o) * inv); }
 
@@ -81,59 +76,101 @@ __device__ __forceinline__ uint32_t fkey(float f) {
     const uint32_t u = __float_as_uint(f);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
-__host__ __forceinline__ float fkey_inv(uint32_t k) {
+__host__ __device__ __forceinline__ float fkey_inv(uint32_t k) {
     const uint32_t u = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(u);
+#else
     float f;
     std::memcpy(&f, &u, 4);
     return f;
+#endif
 }
-__global__ void k_bounds(const float* __restrict__ pos, uint32_t n, uint32_t* __restrict__ bounds) {
+// Bound by its loads in flight and, for small maps, by the atomics on six words: blocks reduce first
+// and a thread reads four photons a turn (100k photons: 14.5 -> 4 us with an atomic per block instead
+// of one per warp).
+__global__ void __launch_bounds__(256) k_bounds(const float* __restrict__ pos, uint32_t n, uint32_t* __restrict__ bounds) {
+    __shared__ uint32_t s_b[6][8];
     uint32_t lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0u, 0u, 0u};
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t step = gridDim.x * blockDim.x;
+    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4u * step) {
+        float v[4][3];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const uint32_t k = fkey(pos[3 * i + a]);
-            lo[a] = min(lo[a], k);
-            hi[a] = max(hi[a], k);
+        for (int u = 0; u < 4; ++u) {
+            const size_t i = min((size_t)i0 + (size_t)u * step, (size_t)n - 1);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) v[u][a] = __ldg(pos + 3 * i + a);
         }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const uint32_t k = fkey(v[u][a]);
+                lo[a] = min(lo[a], k);
+                hi[a] = max(hi[a], k);
+            }
     }
+    const uint32_t warp = threadIdx.x >> 5;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[a] = min(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-            hi[a] = max(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+        lo[a] = __reduce_min_sync(0xffffffffu, lo[a]);
+        hi[a] = __reduce_max_sync(0xffffffffu, hi[a]);
+        if ((threadIdx.x & 31u) == 0) {
+            s_b[a][warp] = lo[a];
+            s_b[3 + a][warp] = hi[a];
         }
     }
-    if ((threadIdx.x & 31u) == 0) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            atomicMin(bounds + a, lo[a]);
-            atomicMax(bounds + 3 + a, hi[a]);
-        }
+    __syncthreads();
+    if (threadIdx.x < 3u) {
+        uint32_t m = 0xffffffffu;
+        for (int w = 0; w < 8; ++w) m = min(m, s_b[threadIdx.x][w]);
+        atomicMin(bounds + threadIdx.x, m);
+    } else if (threadIdx.x < 6u) {
+        uint32_t m = 0u;
+        for (int w = 0; w < 8; ++w) m = max(m, s_b[threadIdx.x][w]);
+        atomicMax(bounds + threadIdx.x, m);
     }
 }
 
-__global__ void k_bucket_count(const float* __restrict__ pos, uint32_t n, BuildParams P, uint32_t* __restrict__ keys,
-                               uint32_t* __restrict__ counts) {
+// One photon of every `stride` counted into the buckets of two trial grids, cells of widths c0 and c1
+// (the density estimate of map_build_impl); the grids' origins follow from the bounds on the device.
+__global__ void k_trial_count(const float* __restrict__ pos, uint32_t n, uint32_t stride, const uint32_t* __restrict__ bounds,
+                              float c0, float c1, uint32_t mask, uint32_t* __restrict__ counts0, uint32_t* __restrict__ counts1) {
+    const uint64_t i = (uint64_t)(blockIdx.x * blockDim.x + threadIdx.x) * stride;
+    if (i >= n) return;
+    float d[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) d[a] = __ldg(pos + 3 * i + a) - fkey_inv(bounds[a]);
+    const float i0 = 1.0f / c0, i1 = 1.0f / c1;
+    // (one cell of margin below the lowest photon, as in the map's own grid)
+    atomicAdd(counts0 + bucket_of((int)floorf((d[0] + c0) * i0), (int)floorf((d[1] + c0) * i0), (int)floorf((d[2] + c0) * i0), mask), 1u);
+    atomicAdd(counts1 + bucket_of((int)floorf((d[0] + c1) * i1), (int)floorf((d[1] + c1) * i1), (int)floorf((d[2] + c1) * i1), mask), 1u);
+}
+
+// The photon's place in its bucket, and the buckets' counts.
+__global__ void k_bucket_rank(const float* __restrict__ pos, uint32_t n, BuildParams P, uint32_t* __restrict__ ranks,
+                              uint32_t* __restrict__ counts) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
+    const float x = pos[3 * (size_t)i], y = pos[3 * (size_t)i + 1], z = pos[3 * (size_t)i + 2];
     const uint32_t b = bucket_of(cell_coord(x, P.ox, P.inv), cell_coord(y, P.oy, P.inv), cell_coord(z, P.oz, P.inv), P.mask);
-    keys[i] = b;
-    atomicAdd(counts + b, 1u);
+    ranks[i] = atomicAdd(counts + b, 1u);
 }
 
-// sum over buckets of count^2 (the photon-weighted bucket occupancy times n)
-__global__ void k_sumsq(const uint32_t* __restrict__ counts, uint32_t nb, unsigned long long* __restrict__ out) {
+// sum over buckets of count^2 (the photon-weighted bucket occupancy times n) of two count arrays
+// (nb each, a multiple of 4)
+__global__ void __launch_bounds__(256) k_sumsq(const uint32_t* __restrict__ counts0, const uint32_t* __restrict__ counts1,
+                                               uint32_t nb, unsigned long long* __restrict__ out) {
+    const uint4* c = reinterpret_cast<const uint4*>(blockIdx.y ? counts1 : counts0);
     unsigned long long s = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += gridDim.x * blockDim.x) {
-        const unsigned long long c = counts[i];
-        s += c * c;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb / 4; i += gridDim.x * blockDim.x) {
+        const uint4 v = c[i];
+        s += (unsigned long long)v.x * v.x + (unsigned long long)v.y * v.y + (unsigned long long)v.z * v.z +
+             (unsigned long long)v.w * v.w;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31u) == 0 && s) atomicAdd(out, s);
+    if ((threadIdx.x & 31u) == 0 && s) atomicAdd(out + blockIdx.y, s);
 }
 
 // exclusive scan of `counts` (n_buckets + 1 entries written to `start`), one block per 1024 x 4 entries
@@ -146,11 +183,18 @@ __global__ void k_scan_local(const uint32_t* __restrict__ in, uint32_t n, uint32
     const uint32_t base = blockIdx.x * kScanBlock * kScanItems + threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
     uint32_t s = 0;
+    if (base + kScanItems <= n) {
+        const uint4 q = *reinterpret_cast<const uint4*>(in + base);
+        v[0] = q.x;
+        v[1] = q.y;
+        v[2] = q.z;
+        v[3] = q.w;
+    } else {
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        v[k] = base + k < n ? in[base + k] : 0u;
-        s += v[k];
+        for (int k = 0; k < kScanItems; ++k) v[k] = base + k < n ? in[base + k] : 0u;
     }
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) s += v[k];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     uint32_t incl = s;
 #pragma unroll
@@ -171,17 +215,34 @@ __global__ void k_scan_local(const uint32_t* __restrict__ in, uint32_t n, uint32
     }
     __syncthreads();
     uint32_t run = incl - s + (warp > 0 ? warp_sums[warp - 1] : 0u);
+    uint32_t e[kScanItems];
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        if (base + k < n) out[base + k] = run;
+        e[k] = run;
         run += v[k];
+    }
+    if (base + kScanItems <= n) {
+        *reinterpret_cast<uint4*>(out + base) = make_uint4(e[0], e[1], e[2], e[3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k)
+            if (base + k < n) out[base + k] = e[k];
     }
     if (threadIdx.x == kScanBlock - 1) block_sums[blockIdx.x] = run;
 }
 
+// (in and out of the scan are 16-byte aligned)
 __global__ void k_scan_add(uint32_t* __restrict__ out, uint32_t n, const uint32_t* __restrict__ block_offsets) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] += block_offsets[i / (kScanBlock * kScanItems)];
+    const uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) * kScanItems;
+    if (base >= n) return;
+    const uint32_t o = block_offsets[base / (kScanBlock * kScanItems)];
+    if (base + kScanItems <= n) {
+        uint4* p = reinterpret_cast<uint4*>(out + base);
+        const uint4 v = *p;
+        *p = make_uint4(v.x + o, v.y + o, v.z + o, v.w + o);
+    } else {
+        for (uint32_t i = base; i < n; ++i) out[i] += o;
+    }
 }
 
 // ---- spatial order of gather queries: a counting sort by the Morton code of a 64^3 grid over the
@@ -207,57 +268,59 @@ __device__ __forceinline__ uint32_t order_key(float x, float y, float z, float o
     return k;
 }
 
-__global__ void k_order_count(const float* __restrict__ q, uint32_t n, float ox, float oy, float oz, float inv,
-                              uint32_t* __restrict__ keys, uint32_t* __restrict__ counts) {
+// the query's place in its cell, and the cells' counts
+__global__ void k_order_rank(const float* __restrict__ q, uint32_t n, float ox, float oy, float oz, float inv,
+                             uint32_t* __restrict__ ranks, uint32_t* __restrict__ counts) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint32_t k = order_key(q[3 * i], q[3 * i + 1], q[3 * i + 2], ox, oy, oz, inv);
-    keys[i] = k;
-    atomicAdd(counts + k, 1u);
+    const size_t j = 3 * (size_t)i;
+    ranks[i] = atomicAdd(counts + order_key(q[j], q[j + 1], q[j + 2], ox, oy, oz, inv), 1u);
 }
 
-__global__ void k_order_scatter(const float* __restrict__ q, uint32_t n, const uint32_t* __restrict__ keys,
-                                uint32_t* __restrict__ cursor, float4* __restrict__ ordered, uint32_t* __restrict__ status) {
+__global__ void k_order_scatter(const float* __restrict__ q, uint32_t n, float ox, float oy, float oz, float inv,
+                                const uint32_t* __restrict__ ranks, const uint32_t* __restrict__ start,
+                                float4* __restrict__ ordered, uint32_t* __restrict__ status) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint32_t slot = atomicAdd(cursor + keys[i], 1u);
+    const size_t j = 3 * (size_t)i;
+    const float x = q[j], y = q[j + 1], z = q[j + 2];
+    const uint32_t slot = start[order_key(x, y, z, ox, oy, oz, inv)] + ranks[i];
     if (slot >= n) {  // cannot happen with consistent counts: record, write nothing
         atomicOr(status, kStatusBadBucket);
         return;
     }
-    ordered[slot] = make_float4(q[3 * i], q[3 * i + 1], q[3 * i + 2], __uint_as_float(i));
+    ordered[slot] = make_float4(x, y, z, __uint_as_float(i));
 }
 
-__global__ void k_scatter(const float* __restrict__ pos, uint32_t n, BuildParams P, const uint32_t* __restrict__ keys,
-                          uint32_t* __restrict__ cursor, float4* __restrict__ sorted, uint64_t* __restrict__ cell_key,
-                          uint32_t* __restrict__ status) {
+// Bound by its random 16-byte writes; the places come from k_bucket_rank, so that no atomic is waited
+// for here.
+__global__ void k_scatter(const float* __restrict__ pos, uint32_t n, BuildParams P, const uint32_t* __restrict__ ranks,
+                          const uint32_t* __restrict__ start, float4* __restrict__ sorted, uint32_t* __restrict__ status) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint32_t slot = atomicAdd(cursor + keys[i], 1u);
+    const float x = pos[3 * (size_t)i], y = pos[3 * (size_t)i + 1], z = pos[3 * (size_t)i + 2];
+    const uint32_t b = bucket_of(cell_coord(x, P.ox, P.inv), cell_coord(y, P.oy, P.inv), cell_coord(z, P.oz, P.inv), P.mask);
+    const uint32_t slot = start[b] + ranks[i];
     if (slot >= n) {  // a bucket range past the photon array: record it, write nothing
         atomicOr(status, kStatusBadBucket);
         return;
     }
-    const float x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
     sorted[slot] = make_float4(x, y, z, __uint_as_float(i));
-    cell_key[slot] = pack_cell(cell_coord(x, P.ox, P.inv), cell_coord(y, P.oy, P.inv), cell_coord(z, P.oz, P.inv));
 }
 
 // bit 31 of a bucket's start marks a bucket that holds photons of more than one cell (hash
 // collisions): the photons of a bucket are contiguous, so two neighbours in the same bucket with
-// different cell keys mark it; the gather checks the cell keys of such buckets photon by photon
-// and those of the other buckets once
+// different cells mark it; the gather checks the cells of such buckets photon by photon and those of
+// the other buckets once
 constexpr uint32_t kBucketMixed = 0x80000000u;
-__device__ __forceinline__ uint32_t bucket_of_key(uint64_t k, uint32_t mask) {
-    const uint32_t m = (1u << kCellBits) - 1u;
-    return bucket_of((int)(uint32_t)(k >> (2 * kCellBits)), (int)((uint32_t)(k >> kCellBits) & m), (int)((uint32_t)k & m), mask);
-}
-__global__ void k_mark_mixed(const uint64_t* __restrict__ cell_key, uint32_t n, uint32_t mask, uint32_t* __restrict__ start) {
+__global__ void k_mark_mixed(const float4* __restrict__ sorted, uint32_t n, BuildParams P, uint32_t* __restrict__ start) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0 || i >= n) return;
-    const uint64_t a = cell_key[i - 1], b = cell_key[i];
-    if (a == b) return;
-    const uint32_t ba = bucket_of_key(a, mask), bb = bucket_of_key(b, mask);
+    const float4 a = sorted[i - 1], b = sorted[i];
+    const int ax = cell_coord(a.x, P.ox, P.inv), ay = cell_coord(a.y, P.oy, P.inv), az = cell_coord(a.z, P.oz, P.inv);
+    const int bx = cell_coord(b.x, P.ox, P.inv), by = cell_coord(b.y, P.oy, P.inv), bz = cell_coord(b.z, P.oz, P.inv);
+    if (ax == bx && ay == by && az == bz) return;
+    const uint32_t ba = bucket_of(ax, ay, az, P.mask), bb = bucket_of(bx, by, bz, P.mask);
     if (ba == bb) atomicOr(start + bb, kBucketMixed);
 }
 
@@ -460,7 +523,7 @@ __device__ __forceinline__ int keep_nearest(uint64_t* buf, int n, int k, int sla
 // photons on surfaces (1M queries, k = 64: 4.96 ms). Here candidates are only filtered by distance and
 // appended, the list is cut to the k nearest two or three times, and sorted once, at the end (2.6 ms,
 // with about seven batches of 32 candidates a query).
-__global__ void __launch_bounds__(256, 4) k_gather(const float4* __restrict__ sorted, const uint64_t* __restrict__ cell_key,
+__global__ void __launch_bounds__(256, 4) k_gather(const float4* __restrict__ sorted,
                                                 const uint32_t* __restrict__ start, GatherParams G,
                                                 const float* __restrict__ queries, uint32_t nq, int k_out,
                                                 int32_t* __restrict__ out_idx, float* __restrict__ out_d2,
@@ -541,7 +604,9 @@ __global__ void __launch_bounds__(256, 4) k_gather(const float4* __restrict__ so
                 }
                 uint32_t s0 = 0, cnt = 0;
                 bool mixed = false;
-                const uint64_t my_key = pack_cell(ix, iy, iz);
+                const auto holds = [&](const float4& p, int x, int y, int z) {  // photon p lies in cell (x, y, z)
+                    return cell_coord(p.x, P.ox, P.inv) == x && cell_coord(p.y, P.oy, P.inv) == y && cell_coord(p.z, P.oz, P.inv) == z;
+                };
                 if (mine) {
                     const uint32_t b = bucket_of(ix, iy, iz, P.mask);
                     const uint32_t r0 = __ldg(start + b);
@@ -552,14 +617,14 @@ __global__ void __launch_bounds__(256, 4) k_gather(const float4* __restrict__ so
                     } else {
                         cnt = s1 - s0;
                         mixed = (r0 & kBucketMixed) != 0u;
-                        // a single-cell bucket: its first key tells whether it is this cell's
-                        if (cnt && !mixed && __ldg(reinterpret_cast<const unsigned long long*>(cell_key) + s0) != my_key) cnt = 0;
+                        // a single-cell bucket: its first photon tells whether it is this cell's
+                        if (cnt && !mixed && !holds(__ldg(sorted + s0), ix, iy, iz)) cnt = 0;
                     }
                 }
                 uint32_t live = __ballot_sync(0xffffffffu, cnt > 0u);
                 if (live == 0u) continue;
                 uint32_t n_live = __popc(live);
-                // mixed buckets are taken one by one, with the cell's key checked photon by photon (and
+                // mixed buckets are taken one by one, with the cell checked photon by photon (and
                 // so are, for the 32-bit prefix sums, buckets of 2^27 photons)
                 const uint32_t slow = __ballot_sync(0xffffffffu, mixed && cnt > 0u) | __ballot_sync(0xffffffffu, cnt >> 27);
                 while (live) {
@@ -575,7 +640,12 @@ __global__ void __launch_bounds__(256, 4) k_gather(const float4* __restrict__ so
                     const float a_d2 = __uint_as_float(ck & ~31u);
                     const uint32_t a_s0 = __shfl_sync(0xffffffffu, s0, src), c_src = __shfl_sync(0xffffffffu, cnt, src);
                     const uint32_t a_cnt = lane < n_live ? c_src : 0u;
-                    const uint64_t target = check ? __shfl_sync(0xffffffffu, (unsigned long long)my_key, src) : 0ull;
+                    int tx = 0, ty = 0, tz = 0;
+                    if (check) {
+                        tx = __shfl_sync(0xffffffffu, ix, src);
+                        ty = __shfl_sync(0xffffffffu, iy, src);
+                        tz = __shfl_sync(0xffffffffu, iz, src);
+                    }
                     // their photons as one list: lane j's cell owns items [excl_j, excl_j + cnt_j), so
                     // that a batch of 32 candidates spans as many cells as it takes
                     uint32_t incl = a_cnt;
@@ -606,7 +676,7 @@ __global__ void __launch_bounds__(256, 4) k_gather(const float4* __restrict__ so
                             const float4 p = __ldg(sorted + i);
                             const float d2 = dist2_exact(p.x, p.y, p.z, qx, qy, qz);
                             key = ((uint64_t)__float_as_uint(d2) << 32) | (uint64_t)__float_as_uint(p.w);
-                            if (check && __ldg(reinterpret_cast<const unsigned long long*>(cell_key) + i) != target) key = INF;
+                            if (check && !holds(p, tx, ty, tz)) key = INF;
                         }
                         const bool better = key < limit;
                         const uint32_t m = __ballot_sync(0xffffffffu, better);
@@ -767,13 +837,17 @@ __global__ void __launch_bounds__(256) k_estimate(const float* __restrict__ powe
 }
 
 int map_build_impl(liar_gpu_ctx* ctx, liar_gpu_photon_map* m, const float* d_pos, size_t n, cudaStream_t st) {
-    // buckets: the next power of two >= 2n, at most 2^23 (the two-level scan covers 2^24 entries)
+    // buckets: the next power of two >= 2n, at most 2^23 (the two-level scan covers 2^24 entries); fewer
+    // below, once the photons are known to lie on surfaces
     uint32_t bits = 10;
     while (bits < 23 && (1ull << bits) < 2ull * n) ++bits;
-    m->bucket_bits = bits;
-    const size_t nb = (size_t)1 << bits;
-    const size_t scan_blocks = (nb + 1 + kScanBlock * kScanItems - 1) / (kScanBlock * kScanItems);
-    const size_t need = n * 4 + 2 * (((nb + 1) * 4 + 255) / 256) * 256 + (scan_blocks + 1) * 8 + 4096;
+    size_t nb = (size_t)1 << bits;
+    size_t scan_blocks = (nb + 1 + kScanBlock * kScanItems - 1) / (kScanBlock * kScanItems);
+    // the density estimate counts one photon in `stride` into at most 2^21 buckets
+    const size_t nb_trial = std::min<size_t>(nb, (size_t)1 << 21);
+    const uint32_t stride = (uint32_t)std::max<size_t>(1, n >> 20);
+    const size_t n_trial = (n + stride - 1) / stride;
+    const size_t need = n * 4 + nb_trial * 4 + (((nb + 1) * 4 + 255) / 256) * 256 + (scan_blocks + 1) * 8 + 4096;
     if (m->scratch_bytes < need) {
         if (m->scratch) cudaFree(m->scratch);
         m->scratch = nullptr;
@@ -789,12 +863,9 @@ int map_build_impl(liar_gpu_ctx* ctx, liar_gpu_photon_map* m, const float* d_pos
     if (m->cap_n < std::max<size_t>(n, 1)) {
         // photons beyond the buffers' capacity (a first build, or a rebuild with more photons)
         if (m->sorted) cudaFree(m->sorted);
-        if (m->cell_key) cudaFree(m->cell_key);
         m->sorted = nullptr;
-        m->cell_key = nullptr;
         m->cap_n = 0;
         e = cudaMalloc((void**)&m->sorted, std::max<size_t>(n, 1) * sizeof(float4));
-        if (e == cudaSuccess) e = cudaMalloc((void**)&m->cell_key, std::max<size_t>(n, 1) * sizeof(uint64_t));
         if (e == cudaSuccess) m->cap_n = std::max<size_t>(n, 1);
     }
     if (e == cudaSuccess && m->cap_buckets < nb + 1) {
@@ -809,16 +880,16 @@ int map_build_impl(liar_gpu_ctx* ctx, liar_gpu_photon_map* m, const float* d_pos
         return ctx_cuda(ctx, e, "photon map");
     }
     char* p = static_cast<char*>(m->scratch);
-    uint32_t* keys = reinterpret_cast<uint32_t*>(p);
+    uint32_t* ranks = reinterpret_cast<uint32_t*>(p);
     p += ((n * 4 + 255) / 256) * 256;
+    uint32_t* counts1 = reinterpret_cast<uint32_t*>(p);  // the second trial grid's, before `counts`
+    p += nb_trial * 4;
     uint32_t* counts = reinterpret_cast<uint32_t*>(p);
-    p += (((nb + 1) * 4 + 255) / 256) * 256;
-    uint32_t* cursor = reinterpret_cast<uint32_t*>(p);
     p += (((nb + 1) * 4 + 255) / 256) * 256;
     uint32_t* bounds = reinterpret_cast<uint32_t*>(p);
     p += 256;
     uint32_t* block_sums = reinterpret_cast<uint32_t*>(p);
-    uint32_t* block_offs = block_sums + scan_blocks + 1;
+    uint32_t* block_offs = block_sums + ((scan_blocks + 4) & ~(size_t)3);  // 16-byte aligned for the scan
     // grid origin and extent from the photons' bounding box
     m->origin[0] = m->origin[1] = m->origin[2] = 0.0f;
     m->extent = 0.0f;
@@ -835,15 +906,29 @@ int map_build_impl(liar_gpu_ctx* ctx, liar_gpu_photon_map* m, const float* d_pos
         return m->extent / cell <= (float)(kCellLimit - 4);
     };
     if (n) {
-        const uint32_t init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-        e = cudaMemcpyAsync(bounds, init, sizeof(init), cudaMemcpyHostToDevice, st);
+        // the bounds and the counts of the density estimate (below) in one go, with one wait for both
+        unsigned long long* d_sum = reinterpret_cast<unsigned long long*>(bounds + 8);
+        e = cudaMemsetAsync(bounds, 0xff, 12, st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(bounds + 3, 0, 36, st);
+        if (e == cudaSuccess && n >= 1024) e = cudaMemsetAsync(counts1, 0, nb_trial * 8, st);
         if (e != cudaSuccess) return ctx_cuda(ctx, e, "photon bounds");
-        const unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)ctx->num_sms * 4);
+        const unsigned blocks = (unsigned)std::min<size_t>((n + 1023) / 1024, (size_t)ctx->num_sms * 4);
         k_bounds<<<blocks, 256, 0, st>>>(d_pos, (uint32_t)n, bounds);
-        uint32_t hb[6];
+        if (n >= 1024) {
+            k_trial_count<<<(unsigned)((n_trial + 255) / 256), 256, 0, st>>>(d_pos, (uint32_t)n, stride, bounds,
+                                                                            m->r_max / 2.0f, m->r_max / 4.0f,
+                                                                            (uint32_t)(nb_trial - 1), counts, counts1);
+            const unsigned sum_blocks = (unsigned)std::min<size_t>((nb_trial / 4 + 255) / 256, (size_t)ctx->num_sms * 4);
+            k_sumsq<<<dim3(sum_blocks, 2), 256, 0, st>>>(counts, counts1, (uint32_t)nb_trial, d_sum);
+        }
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return ctx_cuda(ctx, e, "photon density");
+        uint32_t hb[12];
         e = cudaMemcpyAsync(hb, bounds, sizeof(hb), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return ctx_cuda(ctx, e, "photon bounds");
+        unsigned long long hs[2];
+        std::memcpy(hs, hb + 8, sizeof(hs));
         for (int a = 0; a < 3; ++a) {
             lo[a] = fkey_inv(hb[a]);
             hi[a] = fkey_inv(hb[3 + a]);
@@ -862,26 +947,18 @@ int map_build_impl(liar_gpu_ctx* ctx, liar_gpu_photon_map* m, const float* d_pos
         // 50k photons, 3,000 queries, k = 50: 156, 169, 178, 186 us; cells r_max / 1 .. r_max / 8
         if (n >= 1024) {
             double lam[2] = {0.0, 0.0};
-            unsigned long long* d_sum = reinterpret_cast<unsigned long long*>(bounds + 8);
-            for (int t = 0; t < 2 && e == cudaSuccess; ++t) {
+            for (int t = 0; t < 2; ++t) {
                 if (!set_grid(m->r_max / (t == 0 ? 2.0f : 4.0f))) break;
-                const BuildParams T{m->origin[0], m->origin[1], m->origin[2], 1.0f / m->cell, (uint32_t)(nb - 1)};
-                e = cudaMemsetAsync(counts, 0, nb * 4, st);
-                if (e == cudaSuccess) e = cudaMemsetAsync(d_sum, 0, 8, st);
-                if (e != cudaSuccess) break;
-                k_bucket_count<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_pos, (uint32_t)n, T, keys, counts);
-                k_sumsq<<<(unsigned)ctx->num_sms * 4, 256, 0, st>>>(counts, (uint32_t)nb, d_sum);
-                unsigned long long hs = 0;
-                e = cudaMemcpyAsync(&hs, d_sum, 8, cudaMemcpyDeviceToHost, st);
-                if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-                lam[t] = (double)hs / (double)n - 1.0 - (double)n / (double)nb;
+                lam[t] = ((double)hs[t] / (double)n_trial - 1.0 - (double)n_trial / (double)nb_trial) * (double)stride;
             }
-            if (e != cudaSuccess) return ctx_cuda(ctx, e, "photon density");
             float refine = kRefine;
             if (lam[0] > 0.0 && lam[1] > 0.0) {
                 const double D = std::min(3.0, std::max(1.5, std::log2(lam[0] / lam[1])));
                 const double target = 140.0 * std::pow(9.0 / 140.0, D - 2.0);
                 refine = (float)std::min(8.0, std::max(1.0, 2.0 * std::pow(lam[0] / target, 1.0 / D)));
+                // surfaces: cells of many photons, so that a quarter of the buckets keeps collisions as rare
+                if (target >= 60.0)
+                    while (bits > 10 && (1ull << bits) >= (unsigned long long)n) --bits;
             }
             while (!set_grid(m->r_max / refine) && refine > 1.0f) refine = std::max(1.0f, refine * 0.5f);
         }
@@ -889,24 +966,25 @@ int map_build_impl(liar_gpu_ctx* ctx, liar_gpu_photon_map* m, const float* d_pos
             return ctx_fail(ctx, LIAR_ERR_UNSUPPORTED, "photons span more than %d grid cells per axis; raise r_max",
                             kCellLimit - 4);
     }
+    m->bucket_bits = bits;
+    nb = (size_t)1 << bits;
+    scan_blocks = (nb + 1 + kScanBlock * kScanItems - 1) / (kScanBlock * kScanItems);
     BuildParams P{m->origin[0], m->origin[1], m->origin[2], 1.0f / m->cell, (uint32_t)(nb - 1)};
     e = cudaMemsetAsync(counts, 0, (nb + 1) * 4, st);
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "photon map counts");
-    if (n) k_bucket_count<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_pos, (uint32_t)n, P, keys, counts);
+    if (n) k_bucket_rank<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_pos, (uint32_t)n, P, ranks, counts);
     // exclusive scan of counts[0 .. nb] -> bucket_start (start[nb] = n)
     k_scan_local<<<(unsigned)scan_blocks, kScanBlock, 0, st>>>(counts, (uint32_t)(nb + 1), m->bucket_start, block_sums);
     if (scan_blocks > 1) {
         const size_t blocks2 = (scan_blocks + kScanBlock * kScanItems - 1) / (kScanBlock * kScanItems);
         if (blocks2 > 1) return ctx_fail(ctx, LIAR_ERR_UNSUPPORTED, "photon map too large to scan");
         k_scan_local<<<1, kScanBlock, 0, st>>>(block_sums, (uint32_t)scan_blocks, block_offs, block_sums + scan_blocks);
-        k_scan_add<<<(unsigned)((nb + 1 + 255) / 256), 256, 0, st>>>(m->bucket_start, (uint32_t)(nb + 1), block_offs);
+        k_scan_add<<<(unsigned)((nb + 1 + 1023) / 1024), 256, 0, st>>>(m->bucket_start, (uint32_t)(nb + 1), block_offs);
     }
-    e = cudaMemcpyAsync(cursor, m->bucket_start, (nb + 1) * 4, cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return ctx_cuda(ctx, e, "photon map cursor");
     if (n) {
-        k_scatter<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_pos, (uint32_t)n, P, keys, cursor, m->sorted,
-                                                              m->cell_key, ctx->d_scratch + kStatusWord);
-        k_mark_mixed<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(m->cell_key, (uint32_t)n, (uint32_t)(nb - 1), m->bucket_start);
+        k_scatter<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_pos, (uint32_t)n, P, ranks, m->bucket_start, m->sorted,
+                                                              ctx->d_scratch + kStatusWord);
+        k_mark_mixed<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(m->sorted, (uint32_t)n, P, m->bucket_start);
     }
     m->n = n;
     return ctx_cuda(ctx, cudaGetLastError(), "photon map build");
@@ -985,7 +1063,6 @@ extern "C" void liar_gpu_photon_map_destroy(liar_gpu_photon_map* m) {
     cudaGetDevice(&cur);
     if (m->device >= 0) cudaSetDevice(m->device);
     if (m->sorted) cudaFree(m->sorted);
-    if (m->cell_key) cudaFree(m->cell_key);
     if (m->bucket_start) cudaFree(m->bucket_start);
     if (m->scratch) cudaFree(m->scratch);
     if (cur >= 0) cudaSetDevice(cur);
@@ -1032,29 +1109,27 @@ int order_queries(liar_gpu_ctx* ctx, const liar_gpu_photon_map* m, const float* 
     const size_t scan_blocks = (nb + 1 + kScanBlock * kScanItems - 1) / (kScanBlock * kScanItems);
     const size_t a_ord = ((size_t)n * 16 + 255) / 256 * 256, a_keys = ((size_t)n * 4 + 255) / 256 * 256;
     const size_t a_cnt = ((nb + 1) * 4 + 255) / 256 * 256;
-    int rc = ctx_grow(ctx, &g->mem, &g->cap, a_ord + a_keys + 3 * a_cnt + (scan_blocks + 1) * 8 + 256, "gather order");
+    int rc = ctx_grow(ctx, &g->mem, &g->cap, a_ord + a_keys + 2 * a_cnt + (scan_blocks + 1) * 8 + 256, "gather order");
     if (rc) return rc;
     char* p = static_cast<char*>(g->mem);
     float4* ordered = reinterpret_cast<float4*>(p);
-    uint32_t* keys = reinterpret_cast<uint32_t*>(p + a_ord);
+    uint32_t* ranks = reinterpret_cast<uint32_t*>(p + a_ord);
     uint32_t* counts = reinterpret_cast<uint32_t*>(p + a_ord + a_keys);
     uint32_t* start = reinterpret_cast<uint32_t*>(p + a_ord + a_keys + a_cnt);
-    uint32_t* cursor = reinterpret_cast<uint32_t*>(p + a_ord + a_keys + 2 * a_cnt);
-    uint32_t* block_sums = reinterpret_cast<uint32_t*>(p + a_ord + a_keys + 3 * a_cnt);
-    uint32_t* block_offs = block_sums + scan_blocks + 1;
+    uint32_t* block_sums = reinterpret_cast<uint32_t*>(p + a_ord + a_keys + 2 * a_cnt);
+    uint32_t* block_offs = block_sums + ((scan_blocks + 4) & ~(size_t)3);  // 16-byte aligned for the scan
     cudaError_t e = cudaMemsetAsync(counts, 0, (nb + 1) * 4, st);
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "gather order");
     const float inv = (float)(1 << kOrderBits) / std::max(m->extent, 1e-30f);
     const unsigned blocks = (n + 255) / 256;
-    k_order_count<<<blocks, 256, 0, st>>>(d_q, n, m->origin[0], m->origin[1], m->origin[2], inv, keys, counts);
+    k_order_rank<<<blocks, 256, 0, st>>>(d_q, n, m->origin[0], m->origin[1], m->origin[2], inv, ranks, counts);
     k_scan_local<<<(unsigned)scan_blocks, kScanBlock, 0, st>>>(counts, (uint32_t)(nb + 1), start, block_sums);
     if (scan_blocks > 1) {
         k_scan_local<<<1, kScanBlock, 0, st>>>(block_sums, (uint32_t)scan_blocks, block_offs, block_sums + scan_blocks);
-        k_scan_add<<<(unsigned)((nb + 1 + 255) / 256), 256, 0, st>>>(start, (uint32_t)(nb + 1), block_offs);
+        k_scan_add<<<(unsigned)((nb + 1 + 1023) / 1024), 256, 0, st>>>(start, (uint32_t)(nb + 1), block_offs);
     }
-    e = cudaMemcpyAsync(cursor, start, (nb + 1) * 4, cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return ctx_cuda(ctx, e, "gather order");
-    k_order_scatter<<<blocks, 256, 0, st>>>(d_q, n, keys, cursor, ordered, ctx->d_scratch + kStatusWord);
+    k_order_scatter<<<blocks, 256, 0, st>>>(d_q, n, m->origin[0], m->origin[1], m->origin[2], inv, ranks, start, ordered,
+                                            ctx->d_scratch + kStatusWord);
     e = cudaGetLastError();
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "gather order");
     *out = ordered;
@@ -1091,7 +1166,7 @@ extern "C" int liar_gpu_photon_gather_device(liar_gpu_ctx* ctx, const liar_gpu_p
         if (rc) return rc;
     }
     const unsigned blocks = (unsigned)std::min<size_t>((n_queries + 7) / 8, (size_t)ctx->num_sms * 8);
-    k_gather<<<blocks, 256, 0, st>>>(m->sorted, m->cell_key, m->bucket_start, G, d_queries, (uint32_t)n_queries, k, d_idx,
+    k_gather<<<blocks, 256, 0, st>>>(m->sorted, m->bucket_start, G, d_queries, (uint32_t)n_queries, k, d_idx,
                                      d_d2, d_count, ctx->d_scratch + kStatusWord, ordered);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && order) {

@@ -73,3 +73,30 @@ def test_estimate_sums_every_record(gpu_ctx, k, n, offset):
     # rounding of up to 64 terms of about 1 and of the scale: 64 * 2^-24 of the sum of magnitudes
     bound = (np.abs(P[I]) * use[..., None]).sum(1) * np.where(c > 0, 0.5 / (np.pi * far), 0.0)[:, None] * 70 * 2.0 ** -24 + 1e-12
     assert np.all(np.abs(out.cpu().double().numpy() - ref) <= bound)
+
+
+@pytest.mark.parametrize("n", [1, 3, 1023, 1024, 1025, 5000, 2_100_003])
+@pytest.mark.parametrize("flat", [False, True], ids=["volume", "surface"])
+def test_maps_of_every_size(gpu_ctx, n, flat):
+    """Map builds below and above the density estimate's first size, with sampled photons in it, and over
+    odd counts; a rebuild with fewer photons in the same buffers answers for those alone."""
+    import torch
+    rng = np.random.default_rng(n)
+    p = rng.uniform(-1, 1, (n, 3)).astype(np.float32)
+    if flat:
+        p[:, 1] = 0.25
+    q = np.concatenate([p[:: max(1, n // 150)][:150], rng.uniform(-1, 1, (50, 3)).astype(np.float32)])
+    if flat:
+        q[:, 1] = 0.25
+    r = 1.5 * (60 / max(n, 60)) ** (1 / 2 if flat else 1 / 3)
+    m = PhotonMap(gpu_ctx, p, r_max=r)
+    for count in (n, (n + 1) // 2):
+        if count != n:
+            d = torch.from_numpy(p[:count]).cuda()
+            torch.cuda.synchronize()
+            m.rebuild(d.data_ptr(), count)
+        idx, d2, cnt = m.gather(q, 33)
+        ri, rd, rc = oracle.knn_grid(p[:count], q, 33, r)
+        np.testing.assert_array_equal(cnt, rc)
+        np.testing.assert_array_equal(idx, ri)
+        np.testing.assert_array_equal(d2[ri >= 0].view(np.int32), rd[ri >= 0].view(np.int32))

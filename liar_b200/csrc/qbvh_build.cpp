@@ -307,17 +307,18 @@ struct Collapser {
                 ghi = std::max(ghi, hi[k]);
             }
             const double v0 = plane_value(0), v1 = plane_value(255);
-            float scl = up((float)(((double)ghi - (double)glo) / (v1 - v0)));
-            float org = 0.0f;
+            // the origin below the lowest plane less its value's share, then the step that reaches the
+            // highest plane from it (a lower origin needs a larger step, by less than it went down)
+            double step = ((double)ghi - (double)glo) / (v1 - v0);
+            float org = down((float)((double)glo - v0 * step)), scl = up((float)(((double)ghi - (double)org) / v1));
+            while (std::isfinite(org) && ((double)org + v0 * (double)scl > (double)glo || (double)org + v1 * (double)scl < (double)ghi)) {
+                org = down(org);
+                scl = up((float)(((double)ghi - (double)org) / v1));
+            }
             // (coordinates near the float range's end, beyond what the exact tests can answer, get
             // the whole grid of a point)
-            const bool ok = std::isfinite(scl) && std::isfinite((float)((double)glo - v0 * (double)scl));
-            if (!ok) scl = 0.0f;
-            while (ok) {
-                org = down((float)((double)glo - v0 * (double)scl));
-                if ((double)org + v1 * (double)scl >= (double)ghi) break;
-                scl = up(scl);
-            }
+            const bool ok = std::isfinite(org) && std::isfinite(scl);
+            if (!ok) org = scl = 0.0f;
             q.org[a] = org;
             q.scl[a] = scl;
             uint32_t lw = 0xffffffffu, hw = 0u;

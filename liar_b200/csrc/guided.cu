@@ -97,8 +97,7 @@ __device__ __forceinline__ SampleKey gkey(const GParams& W, uint32_t slot) {
     const uint64_t g = W.first_path + slot;
     SampleKey k;
     k.seed = W.seed;
-    k.pixel = (uint32_t)(g % (uint64_t)W.npix);
-    k.sample = (uint32_t)(g / (uint64_t)W.npix);
+    split_path(g, (uint32_t)W.npix, k.sample, k.pixel);
     k.spp = (uint32_t)W.spp;
     k.mode = W.sampler;
     return k;
@@ -194,8 +193,10 @@ __global__ void __launch_bounds__(128) k_g_prep(DScene S, GQueue in, const liar_
     for (int c = 0; c < 9; ++c) dst[c] = x[c];
 }
 
+// (registers bounded as k_shade's: slit room, 512^2 x 4, 3.75 ms at five blocks an SM, 3.70 at six, 3.73
+// at eight)
 template <bool TEX>
-__global__ void __launch_bounds__(kShadeThreads) k_g_shade(DScene S, GParams W, GPaths P, GQueue in,
+__global__ void __launch_bounds__(kShadeThreads, TEX ? 1 : 6) k_g_shade(DScene S, GParams W, GPaths P, GQueue in,
                                                            const liar_hit* __restrict__ hits, uint32_t n_in, GQueue out,
                                                            const float* __restrict__ gmix) {
     const int lane = threadIdx.x & 31;
@@ -285,14 +286,24 @@ __global__ void __launch_bounds__(kShadeThreads) k_g_shade(DScene S, GParams W, 
                     float3 wd = mk(0, 0, 1);
                     float value = 0.0f, pdf_s = 0.0f, w_mis = 0.0f, p_mix = 0.0f;
                     bool ok = false;
-                    if (sample_dim(key, base + OFF_STRATEGY, strat) < strategy_pdf) {
+                    // the technique, then its sample values, drawn by all lanes together (render.cu)
+                    const bool directional = sample_dim(key, base + OFF_STRATEGY, strat) < strategy_pdf;
+                    const bool by_guide = directional && c > 0.0f && sample_dim(key, gbase, false) < c;
+                    VertexSamples vs;
+                    if (by_guide) {
+                        vs.pick = sample_dim(key, gbase + 1, false);
+                        vs.x = sample_dim(key, gbase + 2, false);
+                        vs.y = sample_dim(key, gbase + 3, false);
+                    } else {
+                        vs = vertex_samples(key, base, strat, directional, B.type, S.n_lights);
+                    }
+                    if (directional) {
                         float p_dir = 0.0f;
-                        if (c > 0.0f && sample_dim(key, gbase, false) < c) {
+                        if (by_guide) {
                             // the guide
                             ++n_guided;
                             float gx, gy, gz;
-                            mixture_sample(mix, sample_dim(key, gbase + 1, false), sample_dim(key, gbase + 2, false),
-                                           sample_dim(key, gbase + 3, false), gx, gy, gz);
+                            mixture_sample(mix, vs.pick, vs.x, vs.y, gx, gy, gz);
                             wd = mk(gx, gy, gz);
                             wo = mk(dot(wd, u), dot(wd, v), dot(wd, N));
                             const BsdfOut be = bsdf_evaluate(B, wi, wo, CAP_ALL);
@@ -300,9 +311,7 @@ __global__ void __launch_bounds__(kShadeThreads) k_g_shade(DScene S, GParams W, 
                             value = be.value;
                             ok = p_dir > 0.0f && value != 0.0f;
                         } else {
-                            const BsdfSample bs = bsdf_sample(B, wi, sample_dim(key, base + OFF_BSDF, strat),
-                                                              sample_dim(key, base + OFF_BSDF + 1, strat),
-                                                              sample_dim(key, base + OFF_COMPONENT, strat), CAP_ALL);
+                            const BsdfSample bs = bsdf_sample(B, wi, vs.x, vs.y, vs.pick, CAP_ALL);
                             if (bs.ok()) {
                                 wo = bs.wo;
                                 wd = bs.wo.x * u + bs.wo.y * v + bs.wo.z * N;
@@ -326,13 +335,11 @@ __global__ void __launch_bounds__(kShadeThreads) k_g_shade(DScene S, GParams W, 
                             p_mix = pdf_s + pl;
                         }
                     } else if (S.n_lights > 0) {
-                        const float uc = sample_dim(key, base + OFF_LIGHT_CHOICE, strat);
-                        int k = lower_bound_f(S.light_cdf, S.n_lights, uc);
+                        int k = lower_bound_f(S.light_cdf, S.n_lights, vs.pick);
                         if (k > S.n_lights - 1) k = S.n_lights - 1;
                         const float pc = light_choice_pdf(S, k);
                         if (pc > 0.0f) {
-                            const LightSample ls = light_sample(S, k, target, sample_dim(key, base + OFF_LIGHT, strat),
-                                                                sample_dim(key, base + OFF_LIGHT + 1, strat), lam);
+                            const LightSample ls = light_sample(S, k, target, vs.x, vs.y, lam);
                             if (ls.pdf > 0.0f) {
                                 float pdf = pc * ls.pdf;
                                 for (int l = 0; l < S.n_lights; ++l) {

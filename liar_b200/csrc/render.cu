@@ -95,8 +95,7 @@ struct WaveParams {
 __device__ __forceinline__ SampleKey key_of(const WaveParams& W, uint64_t gpath) {
     SampleKey k;
     k.seed = W.seed;
-    k.pixel = (uint32_t)(gpath / (uint64_t)W.spp);
-    k.sample = (uint32_t)(gpath % (uint64_t)W.spp);
+    split_path(gpath, (uint32_t)W.spp, k.pixel, k.sample);
     k.spp = (uint32_t)W.spp;
     k.mode = W.sampler;
     return k;
@@ -155,8 +154,10 @@ __global__ void __launch_bounds__(256) k_raygen(DScene S, WaveParams W, Paths P,
 }
 
 // the whole of tracePhoton after the intersection, for one queue entry
+// Waits on chains of dependent loads and instructions (issue slots about half used), so registers are
+// bounded for six blocks an SM (96 -> 80: 256^2 x 16 Cornell frame 982 -> 949 us; 64: 954).
 template <bool TEX>
-__global__ void __launch_bounds__(128) k_shade(DScene S, WaveParams W, Paths P, Queue in, const liar_hit* hits,
+__global__ void __launch_bounds__(128, TEX ? 1 : 6) k_shade(DScene S, WaveParams W, Paths P, Queue in, const liar_hit* hits,
                                                uint32_t n_in, const uint32_t* __restrict__ n_dev, Queue out,
                                                unsigned long long* stats) {
     // n_dev: the queue's size in device memory when the host launched with an upper bound
@@ -236,22 +237,20 @@ __global__ void __launch_bounds__(128) k_shade(DScene S, WaveParams W, Paths P, 
                 int k = -1;
                 float3 dir = mk(0, 0, 1);
                 float acc = 0.0f;
+                const VertexSamples vs = vertex_samples(key, base, strat, by_bsdf, B.type, S.n_lights);
                 if (by_bsdf) {
-                    out = bsdf_sample(B, wi, sample_dim(key, base + OFF_BSDF, strat), sample_dim(key, base + OFF_BSDF + 1, strat),
-                                      sample_dim(key, base + OFF_COMPONENT, strat), CAP_ALL);
+                    out = bsdf_sample(B, wi, vs.x, vs.y, vs.pick, CAP_ALL);
                     if (out.ok()) {
                         out.pdf *= strategy_pdf;
                         dir = out.wo.x * u + out.wo.y * v + out.wo.z * N;
                         have = true;
                     }
                 } else if (S.n_lights > 0) {
-                    const float uc = sample_dim(key, base + OFF_LIGHT_CHOICE, strat);
-                    k = lower_bound_f(S.light_cdf, S.n_lights, uc);
+                    k = lower_bound_f(S.light_cdf, S.n_lights, vs.pick);
                     if (k > S.n_lights - 1) k = S.n_lights - 1;
                     const float pc = light_choice_pdf(S, k);
                     if (pc > 0.0f) {
-                        const LightSample ls = light_sample(S, k, target, sample_dim(key, base + OFF_LIGHT, strat),
-                                                            sample_dim(key, base + OFF_LIGHT + 1, strat), lam);
+                        const LightSample ls = light_sample(S, k, target, vs.x, vs.y, lam);
                         if (ls.pdf > 0.0f) {
                             acc = pc * ls.pdf;
                             dir = ls.dir;

@@ -520,7 +520,10 @@ __device__ inline bool parallelogram_hit(const liar_light& L, float3 o, float3 d
 // SceneLight::emission for a ray leaving `o` along unit `d` (LightArea::doEmission ->
 // SceneObject::doAngularPdf: t^2 / |A cos|; the single-sided test sees a normal already flipped
 // toward the ray's origin, so hits are accepted from both sides)
-__device__ inline LightEmission light_emission(const DScene& S, int li, float3 o, float3 d, float lambda) {
+// radiance(): the light's spectrum at the sample's wavelength (a caller with many samples of a light
+// evaluates it once)
+template <class R>
+__device__ __forceinline__ LightEmission light_emission_of(const DScene& S, int li, float3 o, float3 d, const R& radiance) {
     LightEmission e{0.0f, 0.0f, INFINITY};
     const liar_light L = S.lights[li];
     if (L.type == LIAR_LIGHT_AREA_PARALLELOGRAM) {
@@ -529,7 +532,7 @@ __device__ inline LightEmission light_emission(const DScene& S, int li, float3 o
         const float3 n = normal(cross(mk(L.u[0], L.u[1], L.u[2]), mk(L.v[0], L.v[1], L.v[2])));
         e.pdf = sqr(t) / fabsf(S.light_area[li] * dot(d, n));
         e.t = t;
-        e.value = spec_eval(S, L.spectrum, lambda, false);
+        e.value = radiance();
         return e;
     }
     if (L.type == LIAR_LIGHT_AREA_MESH) {
@@ -555,16 +558,19 @@ __device__ inline LightEmission light_emission(const DScene& S, int li, float3 o
         const float3 n = normal(cross(mk(b[0] - a[0], b[1] - a[1], b[2] - a[2]), mk(c[0] - a[0], c[1] - a[1], c[2] - a[2])));
         e.pdf = sqr(tbest) / fabsf(S.light_area[li] * dot(d, n));
         e.t = tbest;
-        e.value = spec_eval(S, L.spectrum, lambda, false);
+        e.value = radiance();
         return e;
     }
     if (L.type == LIAR_LIGHT_SKY) {
         e.pdf = 1.0f / (4.0f * kPi);
         e.t = S.sky_distance;
-        e.value = spec_eval(S, L.spectrum, lambda, false);
+        e.value = radiance();
         return e;
     }
     return e;  // point lights are never hit
+}
+__device__ inline LightEmission light_emission(const DScene& S, int li, float3 o, float3 d, float lambda) {
+    return light_emission_of(S, li, o, d, [&]() { return spec_eval(S, S.lights[li].spectrum, lambda, false); });
 }
 
 struct LightSample {
@@ -575,7 +581,9 @@ struct LightSample {
 };
 
 // SceneLight::sampleEmission(sample, lightSample, target, shadowRay, pdf)
-__device__ inline LightSample light_sample(const DScene& S, int li, float3 target, float sx, float sy, float lambda) {
+template <class R>
+__device__ __forceinline__ LightSample light_sample_of(const DScene& S, int li, float3 target, float sx, float sy,
+                                                       const R& radiance) {
     LightSample out{mk(0, 0, 1), 0.0f, 0.0f, 0.0f};
     const liar_light L = S.lights[li];
     if (L.type == LIAR_LIGHT_AREA_PARALLELOGRAM || L.type == LIAR_LIGHT_AREA_MESH) {
@@ -621,7 +629,7 @@ __device__ inline LightSample light_sample(const DScene& S, int li, float3 targe
         out.dist = dist;
         if (!L.double_sided && dot(n, tl) > 0.0f) return out;  // target behind a single-sided light
         out.pdf = pdf;
-        out.value = spec_eval(S, L.spectrum, lambda, false);
+        out.value = radiance();
         return out;
     }
     if (L.type == LIAR_LIGHT_POINT) {
@@ -631,7 +639,7 @@ __device__ inline LightSample light_sample(const DScene& S, int li, float3 targe
         out.dir = (1.0f / dist) * tl;
         out.dist = dist;
         out.pdf = 1.0f;
-        out.value = spec_eval(S, L.spectrum, lambda, false) / d2;  // default attenuation 1/d^2
+        out.value = radiance() / d2;  // default attenuation 1/d^2
         return out;
     }
     if (L.type == LIAR_LIGHT_SKY) {
@@ -639,10 +647,41 @@ __device__ inline LightSample light_sample(const DScene& S, int li, float3 targe
         out.dir = uniform_sphere(sx, sy, pdf);
         out.dist = S.sky_distance;
         out.pdf = pdf;
-        out.value = spec_eval(S, L.spectrum, lambda, false);
+        out.value = radiance();
         return out;
     }
     return out;
+}
+__device__ inline LightSample light_sample(const DScene& S, int li, float3 target, float sx, float sy, float lambda) {
+    return light_sample_of(S, li, target, sx, sy, [&]() { return spec_eval(S, S.lights[li].spectrum, lambda, false); });
+}
+
+// The sample values of a vertex that scatters by its BSDF or toward a light. A stratified value costs
+// about 170 integer instructions (seven 64-bit hashes), and drawn inside the two branches each lane of a
+// warp paid for both: the lanes draw their own branch's dimensions together, and only those that the
+// branch reads (the light's choice among several, the component of BSDFs with two, directions where
+// there is a lobe to sample).
+__device__ __forceinline__ bool bsdf_takes_direction(uint32_t type) {
+    return type == LIAR_MAT_LAMBERT || type == LIAR_MAT_COOK_TORRANCE || type == LIAR_MAT_WALTER;
+}
+__device__ __forceinline__ bool bsdf_takes_component(uint32_t type) {
+    return type == LIAR_MAT_DIELECTRIC || type == LIAR_MAT_WALTER;
+}
+struct VertexSamples {
+    float x, y;  // the direction
+    float pick;  // the BSDF's component or the light
+};
+__device__ __forceinline__ VertexSamples vertex_samples(const SampleKey& key, uint32_t base, bool strat, bool by_bsdf,
+                                                        uint32_t type, int n_lights) {
+    VertexSamples v{0.0f, 0.0f, 0.0f};
+    const uint32_t dir = base + (by_bsdf ? (uint32_t)OFF_BSDF : (uint32_t)OFF_LIGHT);
+    if (by_bsdf ? bsdf_takes_direction(type) : n_lights > 0) {
+        v.x = sample_dim(key, dir, strat);
+        v.y = sample_dim(key, dir + 1u, strat);
+    }
+    if (by_bsdf ? bsdf_takes_component(type) : n_lights > 1)
+        v.pick = sample_dim(key, base + (by_bsdf ? (uint32_t)OFF_COMPONENT : (uint32_t)OFF_LIGHT_CHOICE), strat);
+    return v;
 }
 
 __device__ __forceinline__ float light_choice_pdf(const DScene& S, int k) {
@@ -1134,6 +1173,10 @@ __device__ inline Bsdf make_bsdf(const DScene& S, const liar_material& M, const 
 // PerspectiveCamera::doGenerateRay (cameras/perspective_camera.cpp:406-434) for the pixel and
 // sample of key k: stratified jitter in the pixel, thin-lens when the lens radius and focus
 // distance are set; the ray's limits scale the camera's near/far planes by 1 / cos(axis angle)
+__device__ __forceinline__ bool thin_lens(const liar_camera& C) {
+    return C.lens_radius > 0.0f && C.focus_distance > 0.0f && C.focus_distance < 3.4e38f;
+}
+
 // PerspectiveCamera::doGenerateRay at screen point (sx, sy) and lens sample (lu, lv)
 __device__ inline void camera_ray_at(const liar_camera& C, float sx, float sy, float lu, float lv, float3& pos,
                                      float3& dir, float& factor) {
@@ -1143,7 +1186,7 @@ __device__ inline void camera_ray_at(const liar_camera& C, float sx, float sy, f
     dir = normal(dir);
     const float3 dn = mk(C.direction_normal[0], C.direction_normal[1], C.direction_normal[2]);
     factor = 1.0f / dot(dir, dn);
-    if (C.lens_radius > 0.0f && C.focus_distance > 0.0f && C.focus_distance < 3.4e38f) {
+    if (thin_lens(C)) {
         const float2 lens = concentric_disk(lu, lv);
         const float3 lp = pos + (C.lens_radius * lens.x) * mk(C.right_normal[0], C.right_normal[1], C.right_normal[2]) +
                           (C.lens_radius * lens.y) * mk(C.down_normal[0], C.down_normal[1], C.down_normal[2]);
@@ -1154,16 +1197,16 @@ __device__ inline void camera_ray_at(const liar_camera& C, float sx, float sy, f
     }
 }
 
-// screen and lens samples of key k
-__device__ __forceinline__ void camera_samples(const SampleKey& k, int width, int height, float& sx, float& sy,
-                                               float& lu, float& lv) {
+// screen and lens samples of key k (the lens's only where the camera has one)
+__device__ __forceinline__ void camera_samples(const liar_camera& C, const SampleKey& k, int width, int height, float& sx,
+                                               float& sy, float& lu, float& lv) {
     const uint32_t px = k.pixel % (uint32_t)width, py = k.pixel / (uint32_t)width;
     float jx, jy;
     sample_2d(k, DIM_SCREEN, jx, jy);
     sx = ((float)px + jx) / (float)width;
     sy = ((float)py + jy) / (float)height;
     lu = lv = 0.5f;
-    sample_2d(k, DIM_LENS, lu, lv);
+    if (thin_lens(C)) sample_2d(k, DIM_LENS, lu, lv);
 }
 
 // PerspectiveCamera::doGenerateRay (cameras/perspective_camera.cpp:406-434) for the pixel and
@@ -1171,7 +1214,7 @@ __device__ __forceinline__ void camera_samples(const SampleKey& k, int width, in
 // distance are set; the ray's limits scale the camera's near/far planes by 1 / cos(axis angle)
 __device__ inline liar_ray camera_ray(const liar_camera& C, const SampleKey& k, int width, int height) {
     float sx, sy, lu, lv;
-    camera_samples(k, width, height, sx, sy, lu, lv);
+    camera_samples(C, k, width, height, sx, sy, lu, lv);
     float3 pos, dir;
     float factor;
     camera_ray_at(C, sx, sy, lu, lv, pos, dir, factor);
@@ -1184,7 +1227,7 @@ __device__ inline liar_ray camera_ray(const liar_camera& C, const SampleKey& k, 
 __device__ inline void camera_differentials(const liar_camera& C, const SampleKey& k, int width, int height,
                                             float3& oi, float3& di, float3& oj, float3& dj) {
     float sx, sy, lu, lv, f;
-    camera_samples(k, width, height, sx, sy, lu, lv);
+    camera_samples(C, k, width, height, sx, sy, lu, lv);
     const float root = sqrtf((float)k.spp);
     const float dsx = 1.0f / ((float)width * root), dsy = 1.0f / ((float)height * root);
     camera_ray_at(C, sx + dsx, sy, lu, lv, oi, di, f);

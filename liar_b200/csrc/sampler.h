@@ -37,10 +37,15 @@ LS_HD float to_unit(uint64_t h) { return (float)(uint32_t)(h >> 40) * (1.0f / 16
 
 LS_HD uint32_t permute_index(uint32_t i, uint32_t n, uint64_t key) {
     if (n <= 1) return 0;
+    // half of the bits that hold n - 1, rounded up
+#ifdef __CUDA_ARCH__
+    const uint32_t half = (33u - (uint32_t)__clz((int)(n - 1u))) / 2u;
+#else
     uint32_t bits = 0;
-    while ((1u << bits) < n) ++bits;
-    if (bits & 1u) ++bits;
-    const uint32_t half = bits / 2, mask = (1u << half) - 1u;
+    while (bits < 32u && (1ull << bits) < n) ++bits;
+    const uint32_t half = (bits + 1u) / 2u;
+#endif
+    const uint32_t mask = (1u << half) - 1u;
     do {
         uint32_t l = i >> half, r = i & mask;
         for (uint32_t round = 0; round < 4; ++round) {
@@ -91,13 +96,32 @@ LS_HD float dim_jitter(const SampleKey& k, uint64_t hd) {
     return to_unit(mix64(hd + 0xd1b54a32d192ed03ull * ((uint64_t)k.sample + 1)));
 }
 
+// x / n; by a power of two through its exact reciprocal (the same bits as the division)
+LS_HD float over_count(float x, uint32_t n) {
+#ifdef __CUDA_ARCH__
+    if ((n & (n - 1u)) == 0u) return x * __uint_as_float((127u - (31u - (uint32_t)__clz((int)n))) << 23);
+#endif
+    return x / (float)n;
+}
+
+// pixel and sample of path g, spp samples to a pixel
+LS_HD void split_path(uint64_t g, uint32_t spp, uint32_t& pixel, uint32_t& sample) {
+    if (g >> 32) {
+        pixel = (uint32_t)(g / spp);
+        sample = (uint32_t)(g % spp);
+    } else {
+        pixel = (uint32_t)g / spp;
+        sample = (uint32_t)g - pixel * spp;
+    }
+}
+
 LS_HD float sample_dim(const SampleKey& k, uint32_t dim, bool stratified) {
     const uint64_t hd = dim_hash(k, dim);
     if (!stratified) return dim_jitter(k, hd);
     const float jitter = (k.mode & SAMPLER_NOT_JITTERED) ? 0.5f : dim_jitter(k, hd);
     if (k.spp <= 1) return jitter;
     const uint32_t s = permute_index(k.sample, k.spp, hd);
-    const float u = ((float)s + jitter) / (float)k.spp;
+    const float u = over_count((float)s + jitter, k.spp);
     return u < 1.0f ? u : 0.99999994f;
 }
 

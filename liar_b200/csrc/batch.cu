@@ -18,6 +18,8 @@
 
 #include "../../include/liar_gpu.h"
 #include "ctx.h"
+// the scenes lie in device memory here, and the kernels evaluate spectra in a dozen places
+#define LIAR_SPEC_EVAL_ATTR static __noinline__
 #include "render_dev.cuh"
 #include "traverse.cuh"
 
@@ -90,7 +92,7 @@ __device__ __forceinline__ int find_item(const uint64_t* begin, int n, uint64_t 
 }
 
 __device__ __forceinline__ float observer_pdf(const DScene& S, float w) {
-    const int i = upper_bound_f(S.obs_w, S.n_obs, w);
+    const int i = lut_upper_bound(S.luts, S.obs_lut_w, S.obs_w, S.n_obs, w);
     if (i == 0 || i == S.n_obs) return 0.0f;
     return (S.obs_cdf[i] - S.obs_cdf[i - 1]) / (S.obs_w[i] - S.obs_w[i - 1]);
 }
@@ -140,6 +142,7 @@ __device__ void bsplat(const DScene& S, const BItem& it, uint64_t local, const f
     float3 xyz = mk(0, 0, 0);
     if (pdfsum > 0.0f) {
         // balance heuristic over the hero rotations: sum_i L(lam_i) cmf(lam_i) / sum_k p(lam_k)
+#pragma unroll 1
         for (int i = 0; i < H; ++i) {
             const float3 c = observer_sensitivity(S, lam[i]);
             const float s = L[i] / pdfsum;
@@ -197,10 +200,21 @@ __global__ void __launch_bounds__(256) k_b_raygen(BParams P, BState<H> st, BQueu
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&C->stats[0], (unsigned long long)n);
 }
 
-// Waits on chains of dependent loads: eight blocks an SM hide more of them than the spills they take
-// cost (ten scenes, four wavelengths: 11.7 ms at 128 registers, 9.9 at five blocks, 8.9 at eight)
+// adds throughput times spectrum `idx` (-1: nothing) to the path's radiance at every wavelength
+template <int H>
+__device__ __forceinline__ void add_emission(const DScene& S, int idx, const float* T, float* L, const float* lam) {
+    if (idx < 0) return;
+#pragma unroll 1
+    for (int k = 0; k < H; ++k) L[k] += T[k] * spec_eval(S, idx, lam[k], false);
+}
+
+// Waits on chains of dependent loads and on instruction fetch: the path's wavelengths, throughputs and
+// radiances stay in memory, an emission is evaluated in one place, spectra by call and the secondary
+// wavelengths in a loop that is not expanded, and blocks per SM matter more than spills. Ten scenes,
+// four wavelengths, whole batch: 8.9 ms with the four wavelengths expanded and held in registers, then
+// 7.1, 6.8, 6.7 and 6.6 ms at five, six, eight and ten blocks an SM.
 template <int H, bool TEX>
-__global__ void __launch_bounds__(128, TEX ? 1 : 8) k_b_shade(BParams P, BState<H> st, BQueue in, const liar_hit* __restrict__ hits,
+__global__ void __launch_bounds__(128, TEX ? 1 : 10) k_b_shade(BParams P, BState<H> st, BQueue in, const liar_hit* __restrict__ hits,
                                                  int cur, BQueue out) {
     BControl* C = P.ctrl;
     const uint32_t n_in = C->count[cur];
@@ -234,20 +248,20 @@ __global__ void __launch_bounds__(128, TEX ? 1 : 8) k_b_shade(BParams P, BState<
             const int gen_word = st.gen[p];
             const int gen = gen_word & 0xffff;
             bool single = (gen_word >> 16) & 1;
-            float T[H], L[H], lam[H];
-            for (int k = 0; k < H; ++k) {
-                T[k] = st.T[(size_t)H * p + k];
-                L[k] = st.L[(size_t)H * p + k];
-                lam[k] = st.lam[(size_t)H * p + k];
-            }
+            // the path's throughput, radiance and wavelengths stay in memory, read where they are used
+            // (held in registers throughout they were most of what spilled)
+            float* const pT = st.T + (size_t)H * p;
+            float* const pL = st.L + (size_t)H * p;
+            const float* const pl = st.lam + (size_t)H * p;
+            const float lam0 = pl[0];
+            int emission = -1;  // the spectrum that this hit adds
             bool alive = false;
             float3 next_o = mk(0, 0, 0), next_d = mk(0, 0, 1);
             float next_tmin = kTol, next_tmax = INFINITY;
             if (h.prim < 0) {
                 if (S.sky_light >= 0 && S.sky_distance > r0.w * (1.0f + kTol) && S.sky_distance < r1.w * (1.0f - kTol)) {
                     if (gen == 0) st.alpha[p] = 1.0f;
-                    if (gen > 0)
-                        for (int k = 0; k < H; ++k) L[k] += T[k] * spec_eval(S, S.lights[S.sky_light].spectrum, lam[k], false);
+                    if (gen > 0) emission = S.lights[S.sky_light].spectrum;
                 }
             } else {
                 ++n_hit;
@@ -256,8 +270,8 @@ __global__ void __launch_bounds__(128, TEX ? 1 : 8) k_b_shade(BParams P, BState<
                 // the camera vertex carries the camera's ray differentials (texture filtering)
                 if (S.n_tex > 0 && gen == 0) camera_footprint(S, HC, (uint32_t)h.prim, it.cam, key, it.width, it.height);
                 const int light = HC.light, mi = HC.mat;
-                if (gen > 0 && light >= 0)
-                    for (int k = 0; k < H; ++k) L[k] += T[k] * spec_eval(S, S.lights[light].spectrum, lam[k], false);
+                // (a light hit past the camera vertex or the shader's emission, never both)
+                if (gen > 0 && light >= 0) emission = S.lights[light].spectrum;
                 const bool shader_emits = gen == 0 || light < 0;  // as render.cu
                 if (mi < 0) {
                     alive = true;
@@ -266,13 +280,11 @@ __global__ void __launch_bounds__(128, TEX ? 1 : 8) k_b_shade(BParams P, BState<
                     next_tmin = h.t + kTol;
                     next_tmax = r1.w;
                 } else if (S.mats[mi].type == LIAR_MAT_NONE) {
-                    if (shader_emits && S.mats[mi].emission >= 0)
-                        for (int k = 0; k < H; ++k) L[k] += T[k] * spec_eval(S, S.mats[mi].emission, lam[k], false);
+                    if (shader_emits && S.mats[mi].emission >= 0) emission = S.mats[mi].emission;
                 } else {
                     const liar_material M = S.mats[mi];
-                    if (shader_emits && M.emission >= 0)
-                        for (int k = 0; k < H; ++k) L[k] += T[k] * spec_eval(S, M.emission, lam[k], false);
-                    const Bsdf B = make_bsdf<TEX>(S, M, HC, lam[0]);
+                    if (shader_emits && M.emission >= 0) emission = M.emission;
+                    const Bsdf B = make_bsdf<TEX>(S, M, HC, lam0);
                     const float3 md = -d;
                     float3 wi = mk(dot(md, HC.u), dot(md, HC.v), dot(md, HC.N));
                     wi.z = fmaxf(wi.z, kEps);
@@ -293,7 +305,7 @@ __global__ void __launch_bounds__(128, TEX ? 1 : 8) k_b_shade(BParams P, BState<
                             const float3 wd = bs.wo.x * HC.u + bs.wo.y * HC.v + bs.wo.z * HC.N;
                             float pl = 0.0f;
                             for (int l = 0; l < S.n_lights; ++l) {
-                                const LightEmission e = light_emission(S, l, HC.target, wd, lam[0]);
+                                const LightEmission e = light_emission(S, l, HC.target, wd, lam0);
                                 if (e.pdf > 0.0f) pl += light_choice_pdf(S, l) * e.pdf;
                             }
                             pl *= (1.0f - spdf);
@@ -307,12 +319,12 @@ __global__ void __launch_bounds__(128, TEX ? 1 : 8) k_b_shade(BParams P, BState<
                         if (kk > S.n_lights - 1) kk = S.n_lights - 1;
                         const float pc = light_choice_pdf(S, kk);
                         if (pc > 0.0f) {
-                            const LightSample ls = light_sample(S, kk, HC.target, vs.x, vs.y, lam[0]);
+                            const LightSample ls = light_sample(S, kk, HC.target, vs.x, vs.y, lam0);
                             if (ls.pdf > 0.0f) {
                                 float lp = pc * ls.pdf;
                                 for (int l = 0; l < S.n_lights; ++l) {
                                     if (l == kk) continue;
-                                    const LightEmission e = light_emission(S, l, HC.target, ls.dir, lam[0]);
+                                    const LightEmission e = light_emission(S, l, HC.target, ls.dir, lam0);
                                     if (e.pdf > 0.0f) lp += light_choice_pdf(S, l) * e.pdf;
                                 }
                                 lp *= (1.0f - spdf);
@@ -320,6 +332,7 @@ __global__ void __launch_bounds__(128, TEX ? 1 : 8) k_b_shade(BParams P, BState<
                                 const BsdfOut be = bsdf_evaluate(B, wi, lwo, CAP_ALL);
                                 if (be.pdf > 0.0f && be.value != 0.0f) {
                                     wo = lwo;
+                                    bs.value = be.value;
                                     pdf = lp;
                                     w_mis = power_heuristic(lp, be.pdf * spdf);
                                     ok = true;
@@ -327,37 +340,14 @@ __global__ void __launch_bounds__(128, TEX ? 1 : 8) k_b_shade(BParams P, BState<
                             }
                         }
                     }
+                    // (radiance before the throughput changes)
+                    add_emission<H>(S, emission, pT, pL, pl);
+                    emission = -1;
                     if (ok) {
-                        // the BSDF value at every hero wavelength along the chosen direction
                         const bool dispersive = (M.type == LIAR_MAT_DIELECTRIC || M.type == LIAR_MAT_WALTER) &&
                                                 (M.tex[0] >= 0 || M.tex[1] >= 0 ||
                                                  (M.spec[0] >= 0 && S.specs[M.spec[0]].type != LIAR_SPEC_CONSTANT) ||
                                                  (M.spec[1] >= 0 && S.specs[M.spec[1]].type != LIAR_SPEC_CONSTANT));
-                        float val[H];
-                        for (int k = 0; k < H; ++k) {
-                            if (k > 0 && dispersive) {
-                                val[k] = 0.0f;  // secondary wavelengths end at a dispersive interface
-                                continue;
-                            }
-                            const Bsdf Bk = k == 0 ? B : make_bsdf<TEX>(S, M, HC, lam[k]);
-                            if (from_bsdf) {
-                                if (k == 0) {
-                                    val[k] = bs.value;
-                                } else if (Bk.type == LIAR_MAT_CONDUCTOR) {
-                                    val[k] = Bk.r * fresnel_conductor(Bk.eta, Bk.kappa, wi.z) / wi.z;
-                                } else if (Bk.type == LIAR_MAT_MIRROR) {
-                                    val[k] = Bk.r;
-                                } else if (Bk.type == LIAR_MAT_DIELECTRIC) {
-                                    // constant index: same Fresnel, only the reflectance / transmittance differ
-                                    val[k] = wo.z > 0.0f ? bs.value * (B.r != 0.0f ? Bk.r / B.r : 0.0f)
-                                                         : bs.value * (B.t != 0.0f ? Bk.t / B.t : 0.0f);
-                                } else {
-                                    val[k] = bsdf_do_evaluate(Bk, wi, wo, CAP_ALL).value;
-                                }
-                            } else {
-                                val[k] = bsdf_evaluate(Bk, wi, wo, CAP_ALL).value;
-                            }
-                        }
                         const float cos_t = wo.z;
                         next_o = HC.target + ((cos_t > 0.0f ? 10.0f : -10.0f) * kTol) * HC.ng;
                         next_d = wo.x * HC.u + wo.y * HC.v + wo.z * HC.N;
@@ -368,15 +358,60 @@ __global__ void __launch_bounds__(128, TEX ? 1 : 8) k_b_shade(BParams P, BState<
                             // from here on the path exists for lam[0] alone: its later radiance is
                             // weighted by 1 / p(lam[0]) instead of the hero sum 1 / sum_k p(lam[k])
                             // (the splat divides by the sum; radiance gathered so far keeps it)
-                            const float p0 = observer_pdf(S, lam[0]);
+                            const float p0 = observer_pdf(S, lam0);
                             f = p0 > 0.0f ? f * (st.pdfsum[p] / p0) : 0.0f;
                             single = true;
                         }
-                        for (int k = 0; k < H; ++k) T[k] *= val[k] * f;
+                        pT[0] *= bs.value * f;
+                        // the BSDF's value at the other wavelengths along the chosen direction: what does
+                        // not depend on the wavelength (the microfacet terms) once, the rest per
+                        // wavelength in a loop that is not expanded
+                        float shape = 0.0f, cos_h = 0.0f;
+                        if (H > 1 && M.type == LIAR_MAT_COOK_TORRANCE) {
+                            const float3 hv = normal(wi + wo);
+                            float pdfH;
+                            const float dd = mdf_D(B.mdf, hv, B.au, B.av, pdfH);
+                            cos_h = fabsf(dot(wi, hv));
+                            const float gg = fminf(1.0f, fminf(2 * hv.z * wi.z / cos_h, 2 * hv.z * wo.z / cos_h));
+                            shape = dd * gg / (4 * wi.z * wo.z);
+                        }
+#pragma unroll 1
+                        for (int k = 1; k < H; ++k) {
+                            float val = 0.0f;  // secondary wavelengths end at a dispersive interface
+                            if (!dispersive) {
+                                const float lk = pl[k];
+                                if (M.type == LIAR_MAT_LAMBERT) {
+                                    val = param_eval<TEX>(S, M, 0, HC, lk, true) / kPi;
+                                } else if (M.type == LIAR_MAT_WALTER) {
+                                    const Bsdf Bk = make_bsdf<TEX>(S, M, HC, lk);
+                                    val = from_bsdf ? bsdf_do_evaluate(Bk, wi, wo, CAP_ALL).value
+                                                    : bsdf_evaluate(Bk, wi, wo, CAP_ALL).value;
+                                } else if (M.type == LIAR_MAT_DIELECTRIC) {
+                                    // constant index: same Fresnel, only the reflectance / transmittance differ
+                                    const bool up = wo.z > 0.0f;
+                                    const float b0 = up ? B.r : B.t, bk = param_eval<TEX>(S, M, up ? 2 : 3, HC, lk, true);
+                                    val = bs.value * (b0 != 0.0f ? bk / b0 : 0.0f);
+                                } else if (M.type == LIAR_MAT_MIRROR) {
+                                    val = param_eval<TEX>(S, M, 0, HC, lk, true);
+                                } else {
+                                    const float eta = fmaxf(param_eval<TEX>(S, M, 0, HC, lk, false), 1e-9f);
+                                    const float kappa = fmaxf(param_eval<TEX>(S, M, 1, HC, lk, false), 1e-9f);
+                                    const float r = param_eval<TEX>(S, M, 2, HC, lk, true);
+                                    if (M.type == LIAR_MAT_CONDUCTOR) {
+                                        val = r * fresnel_conductor(eta, kappa, wi.z) / wi.z;
+                                    } else {
+                                        val = r * shape;
+                                        val *= fresnel_conductor(eta, kappa, cos_h);
+                                    }
+                                }
+                            }
+                            pT[k] *= val * f;
+                        }
                         alive = true;
                     }
                 }
             }
+            add_emission<H>(S, emission, pT, pL, pl);
             if (alive) {
                 const int ng1 = gen + 1;
                 if (it.max_depth > 0 && ng1 >= it.max_depth) {
@@ -384,21 +419,17 @@ __global__ void __launch_bounds__(128, TEX ? 1 : 8) k_b_shade(BParams P, BState<
                 } else if (ng1 >= it.max_gen) {
                     const float ur = sample_dim(key, DIM_GEN0 + DIMS_PER_GEN * (uint32_t)ng1 + OFF_RR, false);
                     if (ur < 0.5f)
-                        for (int k = 0; k < H; ++k) T[k] /= 0.5f;
+                        for (int k = 0; k < H; ++k) pT[k] /= 0.5f;
                     else
                         alive = false;
                 }
             }
             if (alive) {
-                for (int k = 0; k < H; ++k) {
-                    st.T[(size_t)H * p + k] = T[k];
-                    st.L[(size_t)H * p + k] = L[k];
-                }
                 st.gen[p] = (gen + 1) | (single ? 0x10000 : 0);
                 nr = liar_ray{next_o.x, next_o.y, next_o.z, next_tmin, next_d.x, next_d.y, next_d.z, next_tmax};
                 want = true;
             } else {
-                bsplat<H>(S, it, local, lam, L, st.pdfsum[p], st.alpha[p]);
+                bsplat<H>(S, it, local, pl, pL, st.pdfsum[p], st.alpha[p]);
             }
         }
         bqueue_push(out, &C->count[cur ^ 1], want, nr, p, sc);
@@ -424,12 +455,8 @@ __global__ void __launch_bounds__(256) k_b_flush(BParams P, BState<H> st, BQueue
         const uint32_t p = in.slot[q];
         const BItem& it = P.items[st.item[p]];
         const uint64_t g = (uint64_t)C->wave * P.wave_paths + p;
-        float lam[H], L[H];
-        for (int k = 0; k < H; ++k) {
-            lam[k] = st.lam[(size_t)H * p + k];
-            L[k] = st.L[(size_t)H * p + k];
-        }
-        bsplat<H>(P.scenes[it.scene], it, g - it.path_begin, lam, L, st.pdfsum[p], st.alpha[p]);
+        bsplat<H>(P.scenes[it.scene], it, g - it.path_begin, st.lam + (size_t)H * p, st.L + (size_t)H * p, st.pdfsum[p],
+                  st.alpha[p]);
     }
 }
 

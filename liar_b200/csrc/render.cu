@@ -667,15 +667,52 @@ extern "C" int liar_gpu_scene_upload(liar_gpu_ctx* ctx, const liar_scene_desc* d
     if (!rc) rc = upload(ctx, s, D.materials, D.n_materials, &d.mats, "materials");
     if (!rc) rc = upload(ctx, s, D.spectra, D.n_spectra, &d.specs, "spectra");
     if (!rc) rc = upload(ctx, s, D.spectrum_pool, D.pool_size, &d.pool, "spectrum pool");
-    if (!rc) rc = upload(ctx, s, spec_max.data(), spec_max.size(), &d.spec_max, "spectrum maxima");
     if (!rc) rc = upload(ctx, s, D.lights, D.n_lights, &d.lights, "lights");
     if (!rc) rc = upload(ctx, s, cdf.data(), cdf.size(), &d.light_cdf, "light cdf");
     if (!rc) rc = upload(ctx, s, area.data(), area.size(), &d.light_area, "light areas");
     if (!rc) rc = upload(ctx, s, tri_cdf.data(), tri_cdf.size(), &d.tri_cdf, "mesh light cdf");
-    if (!rc) rc = upload(ctx, s, ow.data(), no, &d.obs_w, "observer");
-    if (!rc) rc = upload(ctx, s, oxyz.data(), 3 * no, &d.obs_xyz, "observer");
-    if (!rc) rc = upload(ctx, s, odxyz.data(), 3 * no, &d.obs_dxyz, "observer");
-    if (!rc) rc = upload(ctx, s, ocdf.data(), no, &d.obs_cdf, "observer");
+    // the spectral tables in one allocation: observer rows, the spectra's search tables and scalars,
+    // the observer's wavelengths and cdf, the search tables
+    const size_t ns = D.n_spectra, at_aux = 8 * no, at_w = at_aux + 4 * ns, at_cdf = at_w + no, at_lut = at_cdf + no;
+    std::vector<float> tab(at_lut);
+    std::vector<uint32_t> luts;
+    for (size_t k = 0; k < no; ++k) {
+        for (int c = 0; c < 3; ++c) {
+            tab[4 * k + c] = oxyz[3 * k + c];
+            tab[4 * (no + k) + c] = odxyz[3 * k + c];
+        }
+        tab[at_w + k] = ow[k];
+        tab[at_cdf + k] = ocdf[k];
+    }
+    for (size_t k = 0; k < ns; ++k) {
+        const liar_spectrum& sp = D.spectra[k];
+        float* a = tab.data() + at_aux + 4 * k;
+        if (sp.type == LIAR_SPEC_SAMPLED) {
+            const SearchLut t = add_lut(luts, D.spectrum_pool + sp.offset, (size_t)sp.count);
+            a[0] = t.x0;
+            a[1] = t.scale;
+            a[2] = spec_max[k];
+            std::memcpy(a + 3, &t.at, sizeof(t.at));
+        } else if (sp.type == LIAR_SPEC_BLACKBODY) {
+            // 1 / Planck's law at the wavelength of its maximum
+            const double T = sp.p[0], w = 2.897771955e-3 / T, h = 6.626070040e-34, c = 299792458.0, kb = 1.3806488e-23;
+            a[2] = (float)(std::pow(w, 5.0) * std::expm1(h * c / kb / (w * T)) / (2 * h * c * c));
+        }
+    }
+    d.obs_lut_w = add_lut(luts, ow.data(), no);
+    d.obs_lut_cdf = add_lut(luts, ocdf.data(), no);
+    tab.resize(at_lut + luts.size());
+    if (!luts.empty()) std::memcpy(tab.data() + at_lut, luts.data(), luts.size() * sizeof(uint32_t));
+    const float* d_tab = nullptr;
+    if (!rc) rc = upload(ctx, s, tab.data(), tab.size(), &d_tab, "spectral tables");
+    if (!rc) {
+        d.obs_xyz = reinterpret_cast<const float4*>(d_tab);
+        d.obs_dxyz = d.obs_xyz + no;
+        d.spec_aux = reinterpret_cast<const float4*>(d_tab + at_aux);
+        d.obs_w = d_tab + at_w;
+        d.obs_cdf = d_tab + at_cdf;
+        d.luts = reinterpret_cast<const uint32_t*>(d_tab + at_lut);
+    }
     if (rc) {
         liar_gpu_scene_destroy(s);
         return rc;

@@ -495,6 +495,7 @@ struct GuidedBuffers {
     uint32_t* counters = nullptr;            // [0] raw records [1] training records [2] candidates
     unsigned long long* stats = nullptr;     // [0..3]
     uint32_t* h_count = nullptr;             // pinned, 4 words
+    cudaEvent_t counted = nullptr;           // the copy of a queue's size into h_count
 };
 
 GuidedBuffers* guided_buffers(liar_gpu_ctx* ctx) {
@@ -505,12 +506,17 @@ GuidedBuffers* guided_buffers(liar_gpu_ctx* ctx) {
     ctx->on_destroy.push_back([gb]() {
         if (gb->mem) cudaFree(gb->mem);
         if (gb->h_count) cudaFreeHost(gb->h_count);
+        if (gb->counted) cudaEventDestroy(gb->counted);
         delete gb;
     });
     return gb;
 }
 
 int ensure_guided_buffers(liar_gpu_ctx* ctx, GuidedBuffers* gb, size_t n, size_t rec_cap) {
+    if (!gb->counted) {
+        cudaError_t e = cudaEventCreateWithFlags(&gb->counted, cudaEventDisableTiming);
+        if (e != cudaSuccess) return ctx_cuda(ctx, e, "guided render event");
+    }
     if (!gb->h_count) {
         cudaError_t e = cudaMallocHost((void**)&gb->h_count, 4 * sizeof(uint32_t));
         if (e != cudaSuccess) return ctx_cuda(ctx, e, "guided render host buffers");
@@ -637,15 +643,23 @@ extern "C" int liar_gpu_render_guided_device(liar_gpu_ctx* ctx, const liar_gpu_s
         if (e == cudaSuccess && train) e = cudaMemsetAsync(gb->counters, 0, 12, st);
         if (e != cudaSuccess) return ctx_cuda(ctx, e, "reset queue");
         k_g_raygen<<<(n + 255) / 256, 256, 0, st>>>(S, W, gb->P, gb->q[0], n);
+        // The trace of a bounce is launched for the size of the bounce before and reads its own on the
+        // device, so that the host learns the queue's size, which the network's launch needs, meanwhile.
         uint32_t n_in = n;
         int cur = 0;
-        for (int bounce = 0; n_in > 0; ++bounce) {
+        for (int bounce = 0;; ++bounce) {
             if (bounce > 4096) return ctx_fail(ctx, LIAR_ERR_TIMEOUT, "paths did not terminate after 4096 bounces");
             if (ctx_cancel_requested(ctx)) return ctx_cancelled(ctx, st);
-            rc = trace_mesh_internal(ctx, mesh, gb->q[cur].rays, n_in, gb->hits, 0, st, kCounterWord + 8);
+            // (the trace clears the size of the queue that the shade kernel fills)
+            rc = trace_mesh_internal(ctx, mesh, gb->q[cur].rays, n_in, gb->hits, 0, st, kCounterWord + 8,
+                                     bounce == 0 ? nullptr : gb->q[cur].count, gb->q[cur ^ 1].count);
             if (rc) return rc;
-            e = cudaMemsetAsync(gb->q[cur ^ 1].count, 0, 4, st);
-            if (e != cudaSuccess) return ctx_cuda(ctx, e, "reset queue");
+            if (bounce > 0) {
+                e = cudaEventSynchronize(gb->counted);
+                if (e != cudaSuccess) return ctx_cuda(ctx, e, "queue size");
+                n_in = gb->h_count[0];
+                if (n_in == 0) break;
+            }
             if (guide_on) {
                 // the guide network over the queue's diffuse and glossy vertices
                 k_g_prep<<<(n_in + 127) / 128, 128, 0, st>>>(S, gb->q[cur], gb->hits, n_in, gb->gin);
@@ -658,9 +672,8 @@ extern "C" int liar_gpu_render_guided_device(liar_gpu_ctx* ctx, const liar_gpu_s
             if (e != cudaSuccess) return ctx_cuda(ctx, e, "guided shade launch");
             cur ^= 1;
             e = cudaMemcpyAsync(gb->h_count, gb->q[cur].count, 4, cudaMemcpyDeviceToHost, st);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+            if (e == cudaSuccess) e = cudaEventRecord(gb->counted, st);
             if (e != cudaSuccess) return ctx_cuda(ctx, e, "queue size");
-            n_in = gb->h_count[0];
         }
         if (train) {
             k_g_finalize<<<ctx->num_sms * 4, 256, 0, st>>>(gb->raw, gb->counters, (uint32_t)rec_cap, gb->P.L, gb->train,

@@ -835,10 +835,10 @@ int render_impl(liar_gpu_ctx* ctx, const liar_gpu_scene* scene, const liar_rende
             if (bounce > 4096) return ctx_fail(ctx, LIAR_ERR_TIMEOUT, "paths did not terminate after 4096 bounces");
             if (ctx_cancel_requested(ctx)) return ctx_cancelled(ctx, st);
             const uint32_t* n_dev = bounce == 0 ? nullptr : rb->q[cur].count;
-            rc = trace_mesh_internal(ctx, scene->mesh, rb->q[cur].rays, bound, rb->hits, 0, st, kCounterWord + 8, n_dev);
+            // (the trace clears the size of the queue that the shade kernel fills)
+            rc = trace_mesh_internal(ctx, scene->mesh, rb->q[cur].rays, bound, rb->hits, 0, st, kCounterWord + 8, n_dev,
+                                     rb->q[cur ^ 1].count);
             if (rc) return rc;
-            e = cudaMemsetAsync(rb->q[cur ^ 1].count, 0, 4, st);
-            if (e != cudaSuccess) return ctx_cuda(ctx, e, "reset queue");
             (S.n_tex > 0 ? k_shade<true> : k_shade<false>)<<<(bound + 127) / 128, 128, 0, st>>>(
                 S, W, rb->P, rb->q[cur], rb->hits, bound, n_dev, rb->q[cur ^ 1], rb->stats);
             e = cudaGetLastError();

@@ -103,7 +103,7 @@ int launch_noalloc(const QNode* nodes, const QTri* tris, const liar_ray* rays, u
     }
     trace_kernel<ANY, kStackNA, kBlockNA, false><<<blocks, kBlockNA, smem, st>>>(
         nodes, tris, rays, hits, n, d.scratch, d.scratch + 1, nullptr,
-        trace_batch(n, blocks * (kBlockNA / 32)), nullptr);
+        trace_batch(n, blocks * (kBlockNA / 32)), nullptr, nullptr);
     if (cudaGetLastError() != cudaSuccess) return LIAR_ERR_CUDA;
     return LIAR_OK;
 }

@@ -556,9 +556,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) trace_kernel(const QNode* __restr
                                                       uint32_t n_rays, uint32_t* __restrict__ work_counter,
                                                       uint32_t* __restrict__ status_word,
                                                       TraceCounters* __restrict__ counters, uint32_t BATCH,
-                                                      const uint32_t* __restrict__ n_dev) {
-    // BATCH: ray indices a warp takes from the global counter at once (trace_batch: n spread over
-    // all resident warps, 32..256, so that a small wave still keeps every warp busy).
+                                                      const uint32_t* __restrict__ n_dev, uint32_t* __restrict__ zero_word) {
+    // BATCH: ray indices a warp takes at once (trace_batch: n spread over all resident warps, at most
+    // 256, so that a small wave still keeps every warp busy).
+    // zero_word: a word that this launch clears (the size of the queue that the next kernel fills), null
+    // for none
+    if (zero_word && blockIdx.x == 0 && threadIdx.x == 0) *zero_word = 0u;
     // n_dev: the ray count in device memory, at most n_rays (a queue whose size the host does not
     // wait for); the launch was sized for n_rays
     if (n_dev) {

@@ -201,8 +201,8 @@ __device__ float record_gradient(const float* o, float wx, float wy, float wz, f
     return -weight * lq;
 }
 
-// ---- inference on tcgen05: four slots of 128 rows per CTA (guide_umma.cuh)
-// Layer 0 runs as four K-chunks over the two halves of the slot's buffer, each chunk committed to
+// ---- inference on tcgen05: slots of 128 rows, six per CTA, four in training (guide_umma.cuh)
+// Layer 0 runs as five K-chunks over the two halves of the slot's buffer, each chunk committed to
 // the half's own mbarrier; a half is rewritten only after the commit of the chunk that read it.
 // Every mbarrier wait is bounded by max_tries polls. A wait that runs out records the timeout,
 // waits once more (bounded again) for every commit still outstanding, so that no MMA still writes
@@ -217,7 +217,7 @@ __device__ float record_gradient(const float* o, float wx, float wy, float wz, f
 // weights normalised by the batch mean from k_weight_sum's block sums, clipped) goes to gout as
 // 48 bf16 (the last 8 zero), the batch loss is added to train[1].
 template <bool TRAIN>
-__global__ void __launch_bounds__(kEvThreads, 1) k_eval_tc(const unsigned char* __restrict__ w_img,
+__global__ void __launch_bounds__(EvShape<TRAIN>::threads, 1) k_eval_tc(const unsigned char* __restrict__ w_img,
                                                            const float* __restrict__ in, size_t n, Box box,
                                                            int stride,
                                                            uint32_t* __restrict__ status, uint32_t max_tries,
@@ -227,31 +227,32 @@ __global__ void __launch_bounds__(kEvThreads, 1) k_eval_tc(const unsigned char* 
                                                            const float* __restrict__ wpart, int n_wpart,
                                                            const __grid_constant__ CUtensorMap tm_store) {
     constexpr int IN = TRAIN ? kRecordFloats : kIn;
+    using E = EvShape<TRAIN>;
     if (TRAIN && n_dev) n = min((size_t)*n_dev, n);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* sw = smem;
-    uint64_t* mbar_all = reinterpret_cast<uint64_t*>(sw + kUmmaWBytes + (size_t)kEvSlots * (kEvBuf + kEvIn));
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbar_all + 2 * kEvSlots);
+    uint64_t* mbar_all = reinterpret_cast<uint64_t*>(sw + kUmmaWBytes + (size_t)E::slots * (E::buf + E::in));
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbar_all + 2 * E::slots);
     volatile uint32_t* failed = tmem_slot + 1;  // one flag per slot
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
     const uint32_t slot = tid >> 7, r = tid & 127u;  // this thread's slot and row within the slot's tile
-    unsigned char* buf = sw + kUmmaWBytes + slot * kEvBuf;
-    float* stage_in = reinterpret_cast<float*>(sw + kUmmaWBytes + (size_t)kEvSlots * kEvBuf + slot * kEvIn);
+    unsigned char* buf = sw + kUmmaWBytes + slot * E::buf;
+    float* stage_in = reinterpret_cast<float*>(sw + kUmmaWBytes + (size_t)E::slots * E::buf + slot * E::in);
     {
         const uint4* s = reinterpret_cast<const uint4*>(w_img);
         uint4* d = reinterpret_cast<uint4*>(sw);
-        for (uint32_t i = tid; i < kUmmaWBytes / 16; i += kEvThreads) d[i] = s[i];
+        for (uint32_t i = tid; i < kUmmaWBytes / 16; i += E::threads) d[i] = s[i];
     }
     if (tid == 0) {
-        for (int k = 0; k < 2 * kEvSlots; ++k)
+        for (int k = 0; k < 2 * E::slots; ++k)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(mbar_all + k)));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        for (int k = 0; k < kEvSlots; ++k) failed[k] = 0u;
+        for (int k = 0; k < E::slots; ++k) failed[k] = 0u;
     }
     if (warp == 0) {
         const uint32_t sa = (uint32_t)__cvta_generic_to_shared(tmem_slot);
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sa), "r"(kEvTmemCols));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sa), "r"(E::tmem_cols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     fence_async_smem();
@@ -316,47 +317,51 @@ __global__ void __launch_bounds__(kEvThreads, 1) k_eval_tc(const unsigned char* 
         return true;
     };
     const size_t n_tiles = (n + kTcRows - 1) / kTcRows;
-    const size_t tile_step = (size_t)gridDim.x * kEvSlots;
+    const size_t tile_step = (size_t)gridDim.x * E::slots;
     bool ok = true;
-    // the inputs of a tile, coalesced: thread r holds elements r + 128 j (j < IN) of the tile's
-    // rows * IN floats; the next tile's are loaded while the current one runs
+    // the next tile's inputs, loaded while the current one runs. Training: coalesced, thread r holds
+    // elements r + 128 j (j < IN) of the tile's rows * IN floats. Inference: row r's nine.
     float pre[IN];
     auto prefetch = [&](size_t t) {
         const size_t base = t * kTcRows * (size_t)IN, end = min(n * (size_t)IN, base + (size_t)kTcRows * IN);
 #pragma unroll
         for (int j = 0; j < IN; ++j) {
-            const size_t i = base + r + 128u * (uint32_t)j;
+            const size_t i = TRAIN ? base + r + 128u * (uint32_t)j : base + (size_t)r * IN + (uint32_t)j;
             pre[j] = (t < n_tiles && i < end) ? __ldg(in + i) : 0.0f;
         }
     };
-    prefetch((size_t)blockIdx.x * kEvSlots + slot);
-    for (size_t tile = (size_t)blockIdx.x * kEvSlots + slot; ok && tile < n_tiles; tile += tile_step) {
+    // (inference: one slot of every CTA before the second of any, so that a few tiles spread out)
+    const size_t first_tile = TRAIN ? (size_t)blockIdx.x * E::slots + slot : (size_t)slot * gridDim.x + blockIdx.x;
+    prefetch(first_tile);
+    for (size_t tile = first_tile; ok && tile < n_tiles; tile += tile_step) {
         const size_t row0 = tile * kTcRows;
         const uint32_t rows = n - row0 < (size_t)kTcRows ? (uint32_t)(n - row0) : (uint32_t)kTcRows;
-        // the tile's inputs through shared memory (the previous tile's readers have passed the slot
-        // barriers since), then the next tile's loads go out
+        // training: the tile's records through shared memory (the previous tile's readers have passed
+        // the slot barriers since), then the next tile's loads go out
+        if (TRAIN) {
 #pragma unroll
-        for (int j = 0; j < IN; ++j) stage_in[r + 128u * (uint32_t)j] = pre[j];
-        prefetch(tile + tile_step);
+            for (int j = 0; j < IN; ++j) stage_in[r + 128u * (uint32_t)j] = pre[j];
+            prefetch(tile + tile_step);
+        }
         if (r == 0) bulk_wait_read();  // the previous tile's last store has read its buffer
         slot_sync();
         float x[kIn];
-        if (r < rows) normalise_input(stage_in + r * IN, box.lo, box.inv_ext, x);
+        if (r < rows) normalise_input(TRAIN ? stage_in + r * IN : pre, box.lo, box.inv_ext, x);
         else
             for (int c = 0; c < kIn; ++c) x[c] = 0.0f;
         // layer 0: chunk c's encodings into half c % 2 once the chunk before last has been consumed
-        uint32_t carry[8];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < kEncChunks; ++c) {
             const int h = c & 1;
             if (c >= 2) wait_half(h);
-            encode_chunk_carry(x, buf + h * kEvHalf, r, c, carry);
-            if (!issue(buf_addr + h * kEvHalf, 1024u, sw_addr + umma_w_offset(0) + 1024u * c, (kEnc / 8) * 128u, 4u,
-                       kWidth, c > 0, h)) {
+            encode_chunk(x, buf + h * E::half, r, c);
+            if (!issue(buf_addr + h * E::half, kChunkCols * 128u, sw_addr + umma_w_offset(0) + kChunkCols * 128u * c,
+                       (kEnc / 8) * 128u, kChunkCols / 2, kWidth, c > 0, h)) {
                 ok = false;
                 break;
             }
         }
+        if (!TRAIN) prefetch(tile + tile_step);
         if (ok) {
             wait_half(0);
             wait_half(1);
@@ -366,16 +371,21 @@ __global__ void __launch_bounds__(kEvThreads, 1) k_eval_tc(const unsigned char* 
             tc_fence_after();
             // training alternates the hidden layers between the halves (h_l in half l % 2), so that
             // the TMA store of one layer's operand runs on while the next layer's is written
-            const uint32_t hh = TRAIN ? (uint32_t)(l & 1) * kEvHalf : 0u;
+            const uint32_t hh = TRAIN ? (uint32_t)(l & 1) * E::half : 0u;
             unsigned char* dst = buf + hh + (r >> 3) * (kWidth / 8) * 128u + (r & 7u) * 16u;
             if (l < kLayers) {
                 // ReLU, bf16, the next layer's A operand (row r, 8 chunks of 8 columns)
-                {
-                    float v[64];
-                    tmem_ld_x64(taddr, v);
+                // (inference: in two reads of 32 columns, for its 80 registers a thread)
+                constexpr int COLS = TRAIN ? 64 : 32;
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const float* q = v + 8 * c;
+                for (int part = 0; part < 64 / COLS; ++part) {
+                    float v[COLS];
+                    if constexpr (TRAIN) tmem_ld_x64(taddr, v);
+                    else tmem_ld_32x32b<32>(taddr + 32u * part, v);
+#pragma unroll
+                    for (int cc = 0; cc < COLS / 8; ++cc) {
+                        const int c = part * (COLS / 8) + cc;
+                        const float* q = v + 8 * cc;
                         // training: rows past the record count hold zeros (they leave with the tile;
                         // their MMA outputs are never read)
                         const uint4 hq = (!TRAIN || r < rows)
@@ -473,10 +483,10 @@ __global__ void __launch_bounds__(kEvThreads, 1) k_eval_tc(const unsigned char* 
     if (r == 0) bulk_wait_all();  // the tile stores are complete before the grid ends
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*tmem_slot), "r"(kEvTmemCols));
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*tmem_slot), "r"(E::tmem_cols));
     if (tid == 0) {
         uint32_t f = 0;
-        for (int k = 0; k < kEvSlots; ++k) f |= failed[k];
+        for (int k = 0; k < E::slots; ++k) f |= failed[k];
         if (f) atomicOr(status, kStatusTimeout);
     }
 }
@@ -1181,9 +1191,9 @@ int smem_attrs(liar_gpu_ctx* ctx) {
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_train_dw_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDwTcSmem);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_eval_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEvSmem);
+        e = cudaFuncSetAttribute(k_eval_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EvShape<false>::smem);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_eval_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEvSmem);
+        e = cudaFuncSetAttribute(k_eval_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EvShape<true>::smem);
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "guide kernel attributes");
     done_device = ctx->device;
     return LIAR_OK;
@@ -1237,12 +1247,12 @@ int guide_train(liar_gpu_ctx* ctx, liar_gpu_guide* G, const float* d_records, co
     const size_t tiles = (n_max + kTcRows - 1) / kTcRows;
     // forward: the inference kernel's four slots storing h_1..h_5, the loss and the output
     // gradient per record
-    const unsigned tgrid = (unsigned)std::max<size_t>(1, std::min<size_t>((tiles + kEvSlots - 1) / kEvSlots, (size_t)sms));
+    const unsigned tgrid = (unsigned)std::max<size_t>(1, std::min<size_t>((tiles + EvShape<true>::slots - 1) / EvShape<true>::slots, (size_t)sms));
     rc = ensure_tensor_maps(ctx, G, n_max);
     if (rc) return rc;
     // the kernels after k_weight_sum start programmatically: each one's prologue (weights to shared
     // memory, barriers, tensor memory) overlaps the end of the kernel before it
-    e = launch_pdl(k_eval_tc<true>, tgrid, kEvThreads, kEvSmem, st, G->umma_w, d_records, n_max, box, 0,
+    e = launch_pdl(k_eval_tc<true>, tgrid, EvShape<true>::threads, EvShape<true>::smem, st, G->umma_w, d_records, n_max, box, 0,
                    status, tries, mma, d_count, n_max, G->scalars, G->gout, (const float*)G->wpart, (int)wgrid,
                    G->tm_act_st);
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "guide training forward");
@@ -1392,7 +1402,7 @@ int liar_gpu::guide::guide_eval(liar_gpu_ctx* ctx, const liar_gpu_guide* G, cons
     if (stride != kOutUsed && stride != kMixRender) return ctx_fail(ctx, LIAR_ERR_INVALID, "mixture stride %d", stride);
     const size_t tiles = (n + kTcRows - 1) / kTcRows;
     if ((uintptr_t)d_mixture & 15u) return ctx_fail(ctx, LIAR_ERR_INVALID, "mixture output not 16-byte aligned");
-    const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>((tiles + kEvSlots - 1) / kEvSlots, (size_t)ctx->num_sms));
+    const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>(tiles, (size_t)ctx->num_sms));
     // the mixtures leave each slot as one TMA store: a 2D map over [n][stride] floats, boxes of
     // 128 rows (rows past n are not written)
     PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
@@ -1407,7 +1417,7 @@ int liar_gpu::guide::guide_eval(liar_gpu_ctx* ctx, const liar_gpu_guide* G, cons
     // the bounded waits' limit: 2^24 polls, far beyond a layer's MMAs; the timeout test
     // (liar_gpu_set_fault_test) issues no MMA and gives up after 2^16 polls
     const bool wait_test = ctx->fault_test == LIAR_FAULT_TEST_GUIDE_WAIT;
-    k_eval_tc<false><<<grid, kEvThreads, kEvSmem, st>>>(G->umma_w, d_inputs, n, make_box(G->cfg), stride,
+    k_eval_tc<false><<<grid, EvShape<false>::threads, EvShape<false>::smem, st>>>(G->umma_w, d_inputs, n, make_box(G->cfg), stride,
                                                           ctx->d_scratch + kStatusWord, wait_test ? 1u << 16 : 1u << 24,
                                                           wait_test ? 0 : 1, nullptr, 0, nullptr, nullptr, nullptr, 0,
                                                           tm_mix);

@@ -53,7 +53,7 @@ __device__ __forceinline__ uint32_t pack_bf16_relu(float lo, float hi) {
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 
-// The encoding of one row as 256 bf16 in a row-major buffer (encode_row_umma of guide_umma.cuh
+// The encoding of one row as 256 bf16 in a row-major buffer (encode_chunk of guide_umma.cuh
 // writes the same values into the K-major operand layout). Per input two sincospi_enc calls (pi x and
 // pi x sqrt(2)); the other frequencies by the doubling formulas sin 2a = 2 sin a cos a,
 // cos 2a = cos^2 a - sin^2 a (x fl(sqrt 2) 2^k is exactly fl(x fl(sqrt 2)) 2^k, so these are the

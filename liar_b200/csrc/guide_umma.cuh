@@ -1,6 +1,6 @@
 // guide_umma.cuh -- the guide network's inference on the 5th-generation tensor cores (tcgen05).
 //
-// A CTA runs four independent 4-warp slots (inference, the training forward and backward), each
+// A CTA runs independent 4-warp slots (six in inference, four in the training forward and backward), each
 // evaluating 128 rows at a time (M = 128; thread r of the slot owns row r), so that one slot's SIMT
 // work overlaps the others' tensor-core work.
 //   * the weights live in shared memory as the B operands of every layer, bf16, K-major, in the
@@ -8,8 +8,8 @@
 //     (n / 8) * (K / 8) * 128 + (k / 8) * 128 + (n % 8) * 16 + (k % 8) * 2 bytes, i.e. 8x16-byte core
 //     matrices with the K-adjacent ones 128 B apart (leading byte offset) and the 8-row groups
 //     (K / 8) * 128 B apart (stride byte offset);
-//   * the activations (A operands) use the same layout: 128 x 256 for the encodings (inference
-//     streams them as four 128 x 64 K-chunks), 128 x 64 for the hidden layers;
+//   * the activations (A operands) use the same layout: the encodings streamed as five 128 x 48
+//     K-chunks, 128 x 64 for the hidden layers;
 //   * a slot's accumulator is 128 lanes x 64 f32 columns of tensor memory; its thread 0 issues each layer
 //     as K / 16 tcgen05.mma (kind::f16, bf16 inputs, f32 accumulation) and commits them to an
 //     mbarrier; every warp then reads its 32 lanes (tcgen05.ld 32x32b.x64), applies ReLU, and
@@ -32,21 +32,33 @@ __host__ __device__ constexpr uint32_t umma_w_offset(int l) {
     return l == 0 ? 0u : (l <= 5 ? 32768u + 8192u * (uint32_t)(l - 1) : 32768u + 4u * 8192u + 6144u);
 }
 constexpr uint32_t kUmmaWBytes = umma_w_offset(6);  // 71680
-constexpr uint32_t kUmmaA0Bytes = (uint32_t)kTcRows * kEnc * 2;    // 65536
 constexpr uint32_t kUmmaA1Bytes = (uint32_t)kTcRows * kWidth * 2;  // 16384
 
-// Inference runs four slots per CTA (16 warps per SM). A slot's operand buffer holds two 128 x 64
-// halves: layer 0's K = 256 is fed to the tensor core in four K-chunks of 64 encodings, chunk c in
-// half c % 2 (the encodings of chunk c + 1 are written while chunk c's MMAs run), and the hidden
-// activations use half 0. After the last layer the buffer stages the slot's 128 output rows (row
-// pitch padded by 4 floats) for coalesced stores; a second area stages the 128 input rows.
-constexpr int kEvSlots = 4;
-constexpr int kEvThreads = 128 * kEvSlots;
-constexpr uint32_t kEvTmemCols = 64 * kEvSlots;
-constexpr uint32_t kEvHalf = (uint32_t)kTcRows * 64 * 2;  // 16384
-constexpr uint32_t kEvBuf = 2 * kEvHalf;                   // 32768
-constexpr uint32_t kEvIn = (uint32_t)kTcRows * 13 * 4;     // 6656: 128 training records of 13 floats
-constexpr size_t kEvSmem = 1024 + kUmmaWBytes + (size_t)kEvSlots * (kEvBuf + kEvIn) + 128;
+// The forward runs slots of 4 warps and 128 rows. Layer 0's encodings are fed to the tensor core in five
+// K-chunks of 48 columns (two inputs' 24 each; the last the ninth input, the raw inputs and zeros: the
+// columns from 240 on are padding and are left out), chunk c in half c % 2 of the slot's operand buffer
+// (the encodings of chunk c + 1 are written while chunk c's MMAs run). The hidden activations take
+// 16 KB of it, the output rows, staged for one TMA store, 128 x 48 floats.
+// Inference: halves of a chunk's size, so that the weights and six slots (24 warps) fit an SM. It waits
+// on tensor memory, barriers and dependent arithmetic with half of the issue slots idle at four slots
+// (chunks of 64 columns, 32 KB buffers): the slots in flight are what bounds it. 2^20 rows: 165 us with
+// four slots, 141 us with six (bytes 37 us, MMAs 45 us at the measured peaks).
+// Training: halves of a whole hidden operand, since a layer's store still reads one while the next is
+// written, and the records' staging rows; four slots.
+constexpr int kEncChunks = 5;
+constexpr uint32_t kChunkCols = 6;  // core columns (8 encodings) of a chunk
+template <bool TRAIN>
+struct EvShape {
+    static constexpr int slots = TRAIN ? 4 : 6;
+    static constexpr int threads = 128 * slots;
+    static constexpr uint32_t tmem_cols = TRAIN ? 256 : 512;  // 64 a slot, a power of two
+    static constexpr uint32_t half = (uint32_t)kTcRows * (TRAIN ? 64 : 8 * kChunkCols) * 2;
+    static constexpr uint32_t buf = 2 * half;
+    static constexpr uint32_t in = TRAIN ? (uint32_t)kTcRows * 13 * 4 : 0;  // 128 training records of 13 floats
+    static constexpr size_t smem = 1024 + kUmmaWBytes + (size_t)slots * (buf + in) + 256;
+};
+static_assert(EvShape<false>::buf >= kUmmaA1Bytes && EvShape<false>::buf >= (uint32_t)kTcRows * 48 * 4, "slot buffer");
+static_assert(EvShape<false>::smem <= 232448 && EvShape<true>::smem <= 232448, "shared memory of a block");
 
 // byte offset of element (row, k) in a K-major no-swizzle operand with K columns
 __host__ __device__ __forceinline__ uint32_t umma_offset(uint32_t row, uint32_t k, uint32_t K) {
@@ -218,118 +230,25 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// the encodings of row r into the 128 x 256 A operand: per input 12 sin/cos pairs = 3 chunks of
-// 16 bytes (angle doubling as encode_row), then the raw inputs and zero padding
-__device__ __forceinline__ void encode_row_umma(const float* x, unsigned char* a0, uint32_t r) {
-    unsigned char* row = a0 + (r >> 3) * (kEnc / 8) * 128u + (r & 7u) * 16u;
+// The K-chunk c (core columns 6 c .. 6 c + 5 of the encodings) of row r into a 128 x 48 K-major operand
+// buffer: per input 12 sin/cos pairs in 3 core columns (encode_input), inputs 2 c and 2 c + 1; in chunk 4
+// the last input, the raw inputs and zeros. No input straddles two chunks.
+__device__ __forceinline__ void encode_chunk(const float* x, unsigned char* a, uint32_t r, int c) {
+    unsigned char* row = a + (r >> 3) * kChunkCols * 128u + (r & 7u) * 16u;
 #pragma unroll
-    for (int d = 0; d < kIn; ++d) {
-        float s0, c0, s1, c1;
-        sincospi_enc(x[d], &s0, &c0);
-        sincospi_enc(x[d] * 1.41421356237309515f, &s1, &c1);
-        uint32_t w[12];
-#pragma unroll
-        for (int k = 0; k < kFreq / 2; ++k) {
-            w[2 * k] = pack_bf16(s0, c0);
-            w[2 * k + 1] = pack_bf16(s1, c1);
-            const float ns0 = 2.0f * s0 * c0, nc0 = c0 * c0 - s0 * s0;
-            const float ns1 = 2.0f * s1 * c1, nc1 = c1 * c1 - s1 * s1;
-            s0 = ns0;
-            c0 = nc0;
-            s1 = ns1;
-            c1 = nc1;
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-            *reinterpret_cast<uint4*>(row + (3 * d + c) * 128u) = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
-    }
-    *reinterpret_cast<uint4*>(row + 27 * 128u) =
-        make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
-    *reinterpret_cast<uint4*>(row + 28 * 128u) = make_uint4(pack_bf16(x[8], 0.0f), 0u, 0u, 0u);
-#pragma unroll
-    for (int c = 29; c < kEnc / 8; ++c) *reinterpret_cast<uint4*>(row + c * 128u) = make_uint4(0u, 0u, 0u, 0u);
-}
-
-// The K-chunk c (encoding columns 64 c .. 64 c + 63) of row r, written into a 128 x 64 K-major
-// operand buffer (the same values as encode_row_umma): the inputs whose 24 columns (3 core
-// columns 3 d .. 3 d + 2) meet the chunk are encoded (an input that straddles two chunks is
-// encoded in both), chunk 3 also holds the raw inputs and the zero padding.
-// The same encodings for the K-chunks of 8 core columns as encode_chunk_umma, every input encoded
-// once: input d fills core columns 3d .. 3d + 2, so inputs 2 (columns 6, 7 | 8) and 5 (15 | 16,
-// 17) straddle a chunk boundary; their columns of the next chunk wait in carry (two columns of four
-// words) and are written by the next call. Calls run for c = 0, 1, 2, 3 in order.
-__device__ __forceinline__ void encode_chunk_carry(const float* x, unsigned char* a, uint32_t r, int c,
-                                                   uint32_t (&carry)[8]) {
-    unsigned char* row = a + (r >> 3) * 8u * 128u + (r & 7u) * 16u;
-    const int lo = 8 * c, hi = 8 * c + 7;  // the chunk's core columns
-    // the columns carried over from the previous chunk: 8 (c = 1), 16 and 17 (c = 2)
-    if (c == 1) *reinterpret_cast<uint4*>(row) = make_uint4(carry[0], carry[1], carry[2], carry[3]);
-    if (c == 2) {
-        *reinterpret_cast<uint4*>(row) = make_uint4(carry[0], carry[1], carry[2], carry[3]);
-        *reinterpret_cast<uint4*>(row + 128) = make_uint4(carry[4], carry[5], carry[6], carry[7]);
-    }
-#pragma unroll
-    for (int d = 0; d < kIn; ++d) {
-        if (3 * d < lo || 3 * d > hi) continue;  // an input belongs to the chunk of its first column
+    for (int d = 2 * c; d < 2 * c + 2 && d < kIn; ++d) {
         uint32_t w[12];
         encode_input(x[d], w);
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            const int col = 3 * d + q;
-            if (col <= hi) {
-                *reinterpret_cast<uint4*>(row + (col - lo) * 128) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-            } else {
-                const int k = col - hi - 1;  // 0 or 1: its slot in the carry
-                carry[4 * k] = w[4 * q];
-                carry[4 * k + 1] = w[4 * q + 1];
-                carry[4 * k + 2] = w[4 * q + 2];
-                carry[4 * k + 3] = w[4 * q + 3];
-            }
-        }
+        for (int q = 0; q < 3; ++q)
+            *reinterpret_cast<uint4*>(row + (3 * (d - 2 * c) + q) * 128u) =
+                make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
     }
-    if (c == 3) {
-        *reinterpret_cast<uint4*>(row + (27 - lo) * 128) =
+    if (c == kEncChunks - 1) {
+        *reinterpret_cast<uint4*>(row + 3 * 128u) =
             make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
-        *reinterpret_cast<uint4*>(row + (28 - lo) * 128) = make_uint4(pack_bf16(x[8], 0.0f), 0u, 0u, 0u);
-#pragma unroll
-        for (int col = 29; col < kEnc / 8; ++col) *reinterpret_cast<uint4*>(row + (col - lo) * 128) = make_uint4(0u, 0u, 0u, 0u);
-    }
-}
-
-__device__ __forceinline__ void encode_chunk_umma(const float* x, unsigned char* a, uint32_t r, int c) {
-    unsigned char* row = a + (r >> 3) * 8u * 128u + (r & 7u) * 16u;
-    const int lo = 8 * c, hi = 8 * c + 7;  // the chunk's core columns
-#pragma unroll
-    for (int d = 0; d < kIn; ++d) {
-        if (3 * d + 2 < lo || 3 * d > hi) continue;
-        float s0, c0, s1, c1;
-        sincospi_enc(x[d], &s0, &c0);
-        sincospi_enc(x[d] * 1.41421356237309515f, &s1, &c1);
-        uint32_t w[12];
-#pragma unroll
-        for (int k = 0; k < kFreq / 2; ++k) {
-            w[2 * k] = pack_bf16(s0, c0);
-            w[2 * k + 1] = pack_bf16(s1, c1);
-            const float ns0 = 2.0f * s0 * c0, nc0 = c0 * c0 - s0 * s0;
-            const float ns1 = 2.0f * s1 * c1, nc1 = c1 * c1 - s1 * s1;
-            s0 = ns0;
-            c0 = nc0;
-            s1 = ns1;
-            c1 = nc1;
-        }
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            const int col = 3 * d + q;
-            if (col >= lo && col <= hi)
-                *reinterpret_cast<uint4*>(row + (col - lo) * 128) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-        }
-    }
-    if (c == 3) {
-        *reinterpret_cast<uint4*>(row + (27 - lo) * 128) =
-            make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
-        *reinterpret_cast<uint4*>(row + (28 - lo) * 128) = make_uint4(pack_bf16(x[8], 0.0f), 0u, 0u, 0u);
-#pragma unroll
-        for (int col = 29; col < kEnc / 8; ++col) *reinterpret_cast<uint4*>(row + (col - lo) * 128) = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(row + 4 * 128u) = make_uint4(pack_bf16(x[8], 0.0f), 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(row + 5 * 128u) = make_uint4(0u, 0u, 0u, 0u);
     }
 }
 

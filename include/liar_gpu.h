@@ -136,6 +136,9 @@ int liar_gpu_mesh_stats(const liar_gpu_mesh* mesh, liar_mesh_stats* out);
  * (src/liar/scenery/triangle_mesh.cpp:321-330): is there a triangle with tmin < t < tmax. */
 int liar_gpu_trace(liar_gpu_ctx* ctx, const liar_gpu_mesh* mesh, const liar_ray* rays, size_t n_rays,
                    liar_hit* hits, int any_hit);
+/* The same with the hits as two host arrays of n_rays elements, apart from each other and the rays. */
+int liar_gpu_trace_columns(liar_gpu_ctx* ctx, const liar_gpu_mesh* mesh, const liar_ray* rays, size_t n_rays,
+                           int32_t* prim, float* t, int any_hit);
 int liar_gpu_trace_device(liar_gpu_ctx* ctx, const liar_gpu_mesh* mesh, const liar_ray* d_rays, size_t n_rays,
                           liar_hit* d_hits, int any_hit, void* stream);
 /* Same as liar_gpu_trace_device, and adds per-ray node visits and triangle tests into

@@ -79,6 +79,7 @@ SIGNATURES: dict[str, tuple] = {
     "liar_gpu_mesh_destroy": (None, [_vp]),
     "liar_gpu_mesh_stats": (C.c_int, [_vp, C.POINTER(MeshStats)]),
     "liar_gpu_trace": (C.c_int, [_vp, _vp, _vp, _sz, _vp, C.c_int]),
+    "liar_gpu_trace_columns": (C.c_int, [_vp, _vp, _vp, _sz, _vp, _vp, C.c_int]),
     "liar_gpu_trace_device": (C.c_int, [_vp, _vp, _vp, _sz, _vp, C.c_int, _vp]),
     "liar_gpu_trace_counted_device": (C.c_int, [_vp, _vp, _vp, _sz, _vp, C.c_int, _vp, _vp]),
     "liar_gpu_trace_device_noalloc": (C.c_int, [_vp, _vp, _sz, _vp, C.c_int, _vp]),

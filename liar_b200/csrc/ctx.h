@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/liar_gpu.h"
+#include "host_stage.h"
 #include "qbvh.h"
 
 namespace liar_gpu {
@@ -40,6 +41,12 @@ struct liar_gpu_ctx {
     cudaStream_t pipe[liar_gpu::kPipeSlots] = {};
     // pipe_ev[k]: end of slot k's work; pipe_ev[kPipeSlots]: start (work queued before the call)
     cudaEvent_t pipe_ev[liar_gpu::kPipeSlots + 1] = {};
+    // pinned staging of the host-buffer trace (host_stage.h; kStageSlots chunks) and its events: a slot's
+    // rays have left it [0], its hits have arrived [1]; rays asked for so far (kStageAfter)
+    void* pin_rays = nullptr;
+    void* pin_hits = nullptr;
+    size_t host_rays = 0;
+    cudaEvent_t stage_ev[2][liar_gpu::kStageSlots] = {};
     // launch shape of the trace kernels (liar_gpu_set_trace_config) and cached occupancy per kernel
     liar_trace_config trace_cfg{128, 16};
     std::unordered_map<const void*, int> occupancy;
@@ -59,6 +66,11 @@ struct liar_gpu_ctx {
             if (pipe[k]) cudaStreamDestroy(pipe[k]);
         for (int k = 0; k <= liar_gpu::kPipeSlots; ++k)
             if (pipe_ev[k]) cudaEventDestroy(pipe_ev[k]);
+        for (auto& slots : stage_ev)
+            for (cudaEvent_t e : slots)
+                if (e) cudaEventDestroy(e);
+        if (pin_rays) cudaFreeHost(pin_rays);
+        if (pin_hits) cudaFreeHost(pin_hits);
     }
 };
 

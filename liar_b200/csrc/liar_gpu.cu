@@ -5,6 +5,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <string>
 
@@ -360,14 +361,129 @@ extern "C" int liar_gpu_trace_counted_device(liar_gpu_ctx* ctx, const liar_gpu_m
                         pick_stream(ctx, stream), ctx->d_scratch + kCounterWord, ctx->d_scratch + kStatusWord);
 }
 
-extern "C" int liar_gpu_trace(liar_gpu_ctx* ctx, const liar_gpu_mesh* mesh, const liar_ray* rays, size_t n_rays,
-                              liar_hit* hits, int any_hit) {
-    if (!ctx) return LIAR_ERR_INVALID;
-    if (!mesh || (n_rays && (!rays || !hits))) return ctx_fail(ctx, LIAR_ERR_INVALID, "null mesh or buffer");
-    if (mesh->device != ctx->device) return ctx_fail(ctx, LIAR_ERR_INVALID, "mesh lives on another device");
-    if (n_rays == 0) return LIAR_OK;
-    int rc = ctx_activate(ctx);
+namespace {
+
+// is p known to CUDA (pinned, registered, managed or device memory)? Copies then run at the link's rate
+// beside the kernels without staging
+bool cuda_memory(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return true;  // left to the copy itself
+    }
+    return a.type != cudaMemoryTypeUnregistered;
+}
+
+// the pinned slots and events for another call of n rays; false: the context has not traced enough rays from
+// host memory yet, or there is no pinned memory to be had
+bool ensure_stage(liar_gpu_ctx* ctx, size_t n) {
+    if (ctx->host_rays < kStageAfter) ctx->host_rays += (n < kStageAfter ? n : kStageAfter) + kStageCall;
+    if (ctx->host_rays < kStageAfter) return false;
+    constexpr size_t rays = kStageSlots * kStageChunk;
+    if (!ctx->pin_rays && cudaHostAlloc(&ctx->pin_rays, rays * sizeof(liar_ray), cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->pin_rays = nullptr;
+        return false;
+    }
+    if (!ctx->pin_hits && cudaHostAlloc(&ctx->pin_hits, rays * sizeof(liar_hit), cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->pin_hits = nullptr;
+        return false;
+    }
+    for (auto& slots : ctx->stage_ev)
+        for (cudaEvent_t& e : slots)
+            if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+                cudaGetLastError();
+                e = nullptr;
+                return false;
+            }
+    return true;
+}
+
+// Trace over pageable rays or hits: chunks of 32,768 rays through the pinned slots, on kPipeSlots streams
+// in turn. Rays or hits in memory known to CUDA are copied directly.
+int trace_staged(liar_gpu_ctx* ctx, const liar_gpu_mesh* mesh, HostStage& stage, bool rays_direct, bool hits_direct,
+                 int any_hit) {
+    const size_t n = stage.n, n_chunks = stage.chunks();
+    const size_t device_rays = n < (size_t)kPipeSlots * kStageChunk ? n : (size_t)kPipeSlots * kStageChunk;
+    int rc = ctx_grow(ctx, &ctx->d_rays, &ctx->cap_rays, device_rays * sizeof(liar_ray), "ray staging buffer");
     if (rc) return rc;
+    rc = ctx_grow(ctx, &ctx->d_hits, &ctx->cap_hits, device_rays * sizeof(liar_hit), "hit staging buffer");
+    if (rc) return rc;
+    rc = ctx_ensure_pipeline(ctx);
+    if (rc) return rc;
+    stage.pin_rays = (liar_ray*)ctx->pin_rays;
+    stage.pin_hits = (liar_hit*)ctx->pin_hits;
+    const size_t n_streams = n_chunks < (size_t)kPipeSlots ? n_chunks : (size_t)kPipeSlots;
+    cudaEventRecord(ctx->pipe_ev[kPipeSlots], ctx->stream);
+    for (size_t s = 0; s < n_streams; ++s) cudaStreamWaitEvent(ctx->pipe[s], ctx->pipe_ev[kPipeSlots], 0);
+    if (!rays_direct) stage.allow_in(kStageSlots);
+    stage.start();
+    size_t issued = 0, left = 0, landed = 0;  // chunks queued, chunks whose rays have left / hits have arrived
+    // lets the copies go on that the device's progress allows, and copies a unit
+    auto work = [&]() {
+        auto advance = [&](cudaEvent_t* ev, size_t* done) {
+            const size_t before = *done;
+            while (!rc && *done < issued) {
+                const cudaError_t e = cudaEventQuery(ev[*done % kStageSlots]);
+                if (e == cudaErrorNotReady) break;
+                if (e != cudaSuccess) rc = ctx_cuda(ctx, e, "trace pipeline");
+                else ++*done;
+            }
+            return *done != before;
+        };
+        if (!rays_direct && advance(ctx->stage_ev[0], &left)) stage.allow_in(left + kStageSlots);
+        if (!hits_direct && advance(ctx->stage_ev[1], &landed)) stage.allow_out(landed);
+        if (!stage.step()) std::this_thread::yield();
+    };
+    for (size_t k = 0; !rc && k < n_chunks; ++k) {
+        const size_t base = k * kStageChunk, m = n - base < kStageChunk ? n - base : kStageChunk;
+        const size_t slot = k % kStageSlots, dev = k % kPipeSlots;
+        if (!rays_direct)
+            while (!rc && !stage.filled(k)) work();
+        if (!hits_direct && k >= kStageSlots)
+            while (!rc && !stage.emptied(k - kStageSlots)) work();
+        if (rc) break;
+        const cudaStream_t st = ctx->pipe[dev];
+        liar_ray* dr = (liar_ray*)ctx->d_rays + dev * kStageChunk;
+        liar_hit* dh = (liar_hit*)ctx->d_hits + dev * kStageChunk;
+        cudaError_t e = cudaMemcpyAsync(dr, rays_direct ? stage.rays + base : stage.pin_rays + slot * kStageChunk,
+                                        m * sizeof(liar_ray), cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaEventRecord(ctx->stage_ev[0][slot], st);
+        if (e != cudaSuccess) {
+            rc = ctx_cuda(ctx, e, "copy rays in");
+            break;
+        }
+        rc = launch_trace(ctx, mesh, dr, m, dh, any_hit, nullptr, st, ctx->d_scratch + kCounterWord + 1 + dev,
+                          ctx->d_scratch + kStatusWord);
+        if (rc) break;
+        e = cudaMemcpyAsync(hits_direct ? stage.hits + base : stage.pin_hits + slot * kStageChunk, dh,
+                            m * sizeof(liar_hit), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaEventRecord(ctx->stage_ev[1][slot], st);
+        if (e != cudaSuccess) {
+            rc = ctx_cuda(ctx, e, "copy hits out");
+            break;
+        }
+        issued = k + 1;
+    }
+    if (!hits_direct)
+        for (size_t k = n_chunks < kStageSlots ? 0 : n_chunks - kStageSlots; !rc && k < n_chunks; ++k)
+            while (!rc && !stage.emptied(k)) work();
+    // work queued on the context stream after this call is ordered after the whole trace
+    for (size_t s = 0; s < n_streams; ++s) {
+        cudaEventRecord(ctx->pipe_ev[s], ctx->pipe[s]);
+        cudaStreamWaitEvent(ctx->stream, ctx->pipe_ev[s], 0);
+    }
+    for (size_t s = 0; s < n_streams; ++s) {
+        const int sync = ctx_cuda(ctx, cudaStreamSynchronize(ctx->pipe[s]), "trace synchronize");
+        if (!rc) rc = sync;
+    }
+    return rc ? rc : ctx_check_status(ctx);
+}
+
+// The copies left to CUDA: at the link's rate from and to pinned memory.
+int trace_unstaged(liar_gpu_ctx* ctx, const liar_gpu_mesh* mesh, const liar_ray* rays, size_t n_rays, liar_hit* hits,
+                   int any_hit) {
     // Chunked pipeline: the copy in of chunk k+1 and the copy out of chunk k-1 overlap the
     // traversal of chunk k (PCIe, not the kernel, bounds this call). Up to kPipeSlots staging
     // slots, each with its own stream and work counter; chunks of 1M rays keep the unoverlapped
@@ -375,7 +491,7 @@ extern "C" int liar_gpu_trace(liar_gpu_ctx* ctx, const liar_gpu_mesh* mesh, cons
     const size_t chunk = n_rays < (size_t)(1u << 20) ? n_rays : (size_t)(1u << 20);
     const size_t n_chunks = (n_rays + chunk - 1) / chunk;
     const int slots = n_chunks < (size_t)kPipeSlots ? (int)n_chunks : kPipeSlots;
-    rc = ctx_grow(ctx, &ctx->d_rays, &ctx->cap_rays, (size_t)slots * chunk * sizeof(liar_ray), "ray staging buffer");
+    int rc = ctx_grow(ctx, &ctx->d_rays, &ctx->cap_rays, (size_t)slots * chunk * sizeof(liar_ray), "ray staging buffer");
     if (rc) return rc;
     rc = ctx_grow(ctx, &ctx->d_hits, &ctx->cap_hits, (size_t)slots * chunk * sizeof(liar_hit), "hit staging buffer");
     if (rc) return rc;
@@ -410,6 +526,50 @@ extern "C" int liar_gpu_trace(liar_gpu_ctx* ctx, const liar_gpu_mesh* mesh, cons
         if (rc) return rc;
     }
     return ctx_check_status(ctx);
+}
+
+}  // namespace
+
+extern "C" int liar_gpu_trace_columns(liar_gpu_ctx* ctx, const liar_gpu_mesh* mesh, const liar_ray* rays, size_t n_rays,
+                                      int32_t* prim, float* t, int any_hit) {
+    if (!ctx) return LIAR_ERR_INVALID;
+    if (!mesh || (n_rays && (!rays || !prim || !t))) return ctx_fail(ctx, LIAR_ERR_INVALID, "null mesh or buffer");
+    if (mesh->device != ctx->device) return ctx_fail(ctx, LIAR_ERR_INVALID, "mesh lives on another device");
+    if (n_rays == 0) return LIAR_OK;
+    int rc = ctx_activate(ctx);
+    if (rc) return rc;
+    if (!ensure_stage(ctx, n_rays)) {  // through interleaved hits and the driver's copies
+        std::unique_ptr<liar_hit[]> hits(new (std::nothrow) liar_hit[n_rays]);
+        if (!hits) return ctx_fail(ctx, LIAR_ERR_OOM, "no memory for %zu hits", n_rays);
+        rc = trace_unstaged(ctx, mesh, rays, n_rays, hits.get(), any_hit);
+        for (size_t i = 0; !rc && i < n_rays; ++i) {
+            prim[i] = hits[i].prim;
+            t[i] = hits[i].t;
+        }
+        return rc;
+    }
+    HostStage stage{rays, nullptr, prim, t, n_rays};
+    return trace_staged(ctx, mesh, stage, cuda_memory(rays), false, any_hit);
+}
+
+extern "C" int liar_gpu_trace(liar_gpu_ctx* ctx, const liar_gpu_mesh* mesh, const liar_ray* rays, size_t n_rays,
+                              liar_hit* hits, int any_hit) {
+    if (!ctx) return LIAR_ERR_INVALID;
+    if (!mesh || (n_rays && (!rays || !hits))) return ctx_fail(ctx, LIAR_ERR_INVALID, "null mesh or buffer");
+    if (mesh->device != ctx->device) return ctx_fail(ctx, LIAR_ERR_INVALID, "mesh lives on another device");
+    if (n_rays == 0) return LIAR_OK;
+    int rc = ctx_activate(ctx);
+    if (rc) return rc;
+    // Pageable rays or hits go through the staging slots. Memory known to CUDA needs none, and rays and hits
+    // that overlap keep their order of copies.
+    const bool rays_direct = cuda_memory(rays), hits_direct = cuda_memory(hits);
+    const uintptr_t ra = (uintptr_t)rays, ha = (uintptr_t)hits;
+    const bool overlap = ra < ha + n_rays * sizeof(liar_hit) && ha < ra + n_rays * sizeof(liar_ray);
+    if (!(rays_direct && hits_direct) && !overlap && ensure_stage(ctx, n_rays)) {
+        HostStage stage{rays, hits, nullptr, nullptr, n_rays};
+        return trace_staged(ctx, mesh, stage, rays_direct, hits_direct, any_hit);
+    }
+    return trace_unstaged(ctx, mesh, rays, n_rays, hits, any_hit);
 }
 
 extern "C" int liar_gpu_set_fault_test(liar_gpu_ctx* ctx, int mode) {

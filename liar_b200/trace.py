@@ -115,10 +115,10 @@ class Mesh:
     def intersect(self, rays: np.ndarray, any_hit: bool = False) -> tuple[np.ndarray, np.ndarray]:
         """Traces host rays; returns (prim, t) host arrays."""
         rays = _as_rays(rays)
-        hits = np.empty((rays.shape[0], 2), dtype=np.int32)
-        self.ctx.check(self.ctx._lib.liar_gpu_trace(self.ctx.handle, self.handle, rays.ctypes.data, rays.shape[0],
-                                                    hits.ctypes.data, int(bool(any_hit))))
-        return hits[:, 0].copy(), hits[:, 1].view(np.float32).copy()
+        prim, t = np.empty(rays.shape[0], dtype=np.int32), np.empty(rays.shape[0], dtype=np.float32)
+        self.ctx.check(self.ctx._lib.liar_gpu_trace_columns(self.ctx.handle, self.handle, rays.ctypes.data, rays.shape[0],
+                                                            prim.ctypes.data, t.ctypes.data, int(bool(any_hit))))
+        return prim, t
 
     def trace_into(self, rays_ptr: int, n: int, hits_ptr: int, any_hit: bool = False, stream: int | None = None,
                    counters_ptr: int | None = None) -> None:

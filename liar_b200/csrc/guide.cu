@@ -521,7 +521,7 @@ __global__ void k_weight_sum(const float* __restrict__ rec, const uint32_t* __re
 
 // ---- training on tcgen05 (guide_umma.cuh's operand layouts and instruction forms)
 //
-// forward  k_eval_tc<true>: the inference kernel's four 4-warp slots of 128 records; after every
+// forward  k_eval_tc<true>: the inference kernel with four 4-warp slots of 128 records; after every
 //          hidden layer its ReLU'd bf16 activations also go to global memory (h_1..h_5, for the
 //          backward masks and the weight gradients); its output layer ends in the loss head (the
 //          loss and its gradient per record, record_gradient), stored bf16
@@ -1245,7 +1245,7 @@ int guide_train(liar_gpu_ctx* ctx, liar_gpu_guide* G, const float* d_records, co
     const int mma = wait_test ? 0 : 1;
     uint32_t* status = ctx->d_scratch + kStatusWord;
     const size_t tiles = (n_max + kTcRows - 1) / kTcRows;
-    // forward: the inference kernel's four slots storing h_1..h_5, the loss and the output
+    // forward: the inference kernel with four slots, storing h_1..h_5, the loss and the output
     // gradient per record
     const unsigned tgrid = (unsigned)std::max<size_t>(1, std::min<size_t>((tiles + EvShape<true>::slots - 1) / EvShape<true>::slots, (size_t)sms));
     rc = ensure_tensor_maps(ctx, G, n_max);

@@ -41,8 +41,9 @@ constexpr uint32_t kUmmaA1Bytes = (uint32_t)kTcRows * kWidth * 2;  // 16384
 // 16 KB of it, the output rows, staged for one TMA store, 128 x 48 floats.
 // Inference: halves of a chunk's size, so that the weights and six slots (24 warps) fit an SM. It waits
 // on tensor memory, barriers and dependent arithmetic with half of the issue slots idle at four slots
-// (chunks of 64 columns, 32 KB buffers): the slots in flight are what bounds it. 2^20 rows: 165 us with
-// four slots, 141 us with six (bytes 37 us, MMAs 45 us at the measured peaks).
+// (chunks of 64 columns, 32 KB buffers): the slots in flight are what bounds it. 10^6 rows: 165 us with
+// four slots, 141 us with six (bytes 30 us, MMAs 40 us at the measured peaks); 10^5: 31 and 23; where
+// whole rounds of four-slot tiles come out even (75,776 rows), 19.4 and 19.8.
 // Training: halves of a whole hidden operand, since a layer's store still reads one while the next is
 // written, and the records' staging rows; four slots.
 constexpr int kEncChunks = 5;
